@@ -386,6 +386,24 @@ bool make_prim_map(eu3d_handle *h)
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// FP64 flux launch: tiles of 32 x 7 columns, two blocks of 8 warps per SM (128
+// registers a thread) where the grid fills the GPU; where it does not, 32 x 3
+// tiles, whose shorter blocks spread over more SMs (on a cheaper limiter, 7 -> 3
+// rows: 241 x 81 x 2 15.2 -> 13.1 us a launch, 4000 x 2 x 2 15.0 -> 11.2, but
+// 160^3 0.56 -> 0.60 ms; with this one 17.3, 13.1 us and 0.75 ms, from 86.6, 78.4
+// us and 6.4 ms before the division-free faces).
+template <int DIFF, bool SQ, int TY, int NB>
+void launch_flux64(eu3d_handle *h, const FluxSolid &wedge)
+{
+    const Layout &L = h->L;
+    const int kz = h->flux_kz;
+    FieldBase qf;
+    for (int f = 0; f < NPRIM; f++) qf.p[f] = (const char *)((const double *)h->prim + f * L.fs);
+    const dim3 g((L.ni + FT_X - 1) / FT_X, (L.nj + TY - 1) / TY, (L.nk + kz - 1) / kz);
+    k_flux64<DIFF, SQ, TY, NB><<<g, dim3(FT_X, TY + 1), Flux64<TY>::SMEM, h->st>>>(L, qf, h->xn, h->yn, h->zn, h->scal,
+                                                                                  (double *)h->rhs, kz, wedge);
+}
+
 template <class P, int DIFF>
 void launch_adv_t(eu3d_handle *h)
 {
@@ -393,12 +411,14 @@ void launch_adv_t(eu3d_handle *h)
     const Layout &L = h->L;
     const int kz = h->flux_kz;
     const FluxSolid wedge{h->wedge[0], h->wedge[1], h->wedge[2], h->wedge_on};
-    constexpr int TY = FluxTile<P>::TY;
-    dim3 g((L.ni + FT_X - 1) / FT_X, (L.nj + TY - 1) / TY, (L.nk + kz - 1) / kz);
-    dim3 b(FT_X, TY + 2);
-    constexpr size_t smem = FluxTile<P>::SMEM;
     ProfScope ps(h, "advection");
-    if constexpr (sizeof(P) == 4) {
+    if constexpr (sizeof(P) == 8) {
+        const long long blocks = (long long)((L.ni + FT_X - 1) / FT_X) * ((L.nj + 6) / 7) * ((L.nk + kz - 1) / kz);
+        if (blocks < 2 * 148)
+            sq ? launch_flux64<DIFF, true, 3, 4>(h, wedge) : launch_flux64<DIFF, false, 3, 4>(h, wedge);
+        else
+            sq ? launch_flux64<DIFF, true, 7, 2>(h, wedge) : launch_flux64<DIFF, false, 7, 2>(h, wedge);
+    } else {
         const float *qf = (const float *)h->prim;
         if (h->flux_stage == 2 && h->tq_ok) {
             dim3 gs((L.ni + FT_X - 1) / FT_X, (L.nj + FR_TY - 1) / FR_TY, (L.nk + kz - 1) / kz);
@@ -418,9 +438,10 @@ void launch_adv_t(eu3d_handle *h)
                                                                    kz, wedge);
             return;
         }
+        dim3 g((L.ni + FT_X - 1) / FT_X, (L.nj + FluxTile::TY - 1) / FluxTile::TY, (L.nk + kz - 1) / kz);
+        k_flux_tile<DIFF><<<g, dim3(FT_X, FluxTile::TY + 2), FluxTile::SMEM, h->st>>>(L, qf, h->xn, h->yn, h->zn, h->scal,
+                                                                                  (float *)h->rhs, sq, kz, wedge);
     }
-    k_flux_tile<P, DIFF><<<g, b, smem, h->st>>>(L, (const P *)h->prim, h->xn, h->yn, h->zn, h->scal, (P *)h->rhs, sq,
-                                                kz, wedge);
 }
 
 template <class P>
@@ -444,10 +465,10 @@ void flux_attributes()
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     }
     cudaFuncSetAttribute(k_flux_stage<DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FluxStage::SMEM);
-    cudaFuncSetAttribute(k_flux_tile<float, DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)FluxTile<float>::SMEM);
-    cudaFuncSetAttribute(k_flux_tile<double, DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)FluxTile<double>::SMEM);
+    cudaFuncSetAttribute(k_flux_tile<DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FluxTile::SMEM);
+    for (auto k : {k_flux64<DIFF, false, 7, 2>, k_flux64<DIFF, true, 7, 2>})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Flux64<7>::SMEM);
+    static_assert(Flux64<3>::SMEM <= 48 * 1024, "the small tile fits the default shared memory");
 }
 
 int adv_op(eu3d_handle *h, int timeadv, int diff)
@@ -1067,6 +1088,17 @@ int eu3d_create(const eu3d_desc *d, eu3d_handle **out)
         const long long cols = (long long)((L.ni + 31) / 32) * ((L.nj + 7) / 8);
         int kz = 64;
         while (kz > 4 && cols * ((L.nk + kz - 1) / kz) < 4LL * 2 * 148) kz /= 2;
+        if (d->flux_bits == 64) {
+            // FP64: a walk of 16 planes already hides its extra z face (240 x
+            // 256 x 200: 2.32 ms, 2.43 with 4 planes, 2.91 with 1); shorter
+            // ones while the 32 x 7 tiles leave fewer than two waves, down to
+            // one plane (160^3: 0.75 ms with 4, 0.77 with 16; 121 x 81 x 61:
+            // 139 us with 2 or 4, 155 with 1; 241 x 81 x 2: 17.3 us with 1,
+            // 21.0 with 2)
+            const long long c7 = (long long)((L.ni + 31) / 32) * ((L.nj + 6) / 7);
+            kz = 16;
+            while (kz > 1 && c7 * ((L.nk + kz - 1) / kz) < 2LL * 2 * 148) kz /= 2;
+        }
         h->flux_kz = kz;
     }
     if ((long long)NPRIM * L.fs >= (1LL << 31)) {

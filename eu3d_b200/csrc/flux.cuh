@@ -7,12 +7,12 @@
 //
 // The reference materialises left/right states of 16 primitives per
 // direction into full-size arrays, then face fluxes F, G, Q, then RHS.  Here
-// no intermediate array exists: k_flux_tile computes each face flux once per
+// no intermediate array exists: each kernel computes each face flux once per
 // step (x and y faces of a block's tile through shared memory, z faces in
 // registers while the block walks its z planes) and writes only the residual
 //     RHS = -dt/dx (F_i - F_{i-1}) - dt/dy (G_j - G_{j-1}) - dt/dz (Q_k - Q_{k-1})
-// accumulated in FP64 in the reference's operation order.  Reconstruction
-// and AUSM run in P (double or float); differences and the residual in FP64.
+// in the reference's operation order.  k_flux64 works in FP64 throughout, the
+// others in FP32.
 #pragma once
 
 #include <cuda.h>
@@ -22,11 +22,50 @@
 
 namespace eu3d {
 
-template <class P>
-__device__ __forceinline__ P minmod_lim(P R)
+// FP64 quotients and square roots without the compiler's out-of-line paths:
+// the hardware's approximation, one third-order step (the approximation's
+// error cubed, below 2^-60) and Markstein's final correction by the exact
+// remainder (P. Markstein, IBM J. Res. Dev. 34, 1990), which rounds as IEEE
+// division and square root do for results and reciprocals in the normal range.
+// Zero, infinite or NaN divisors give NaN.
+__device__ __forceinline__ double rcp_approx(double x)
 {
-    // Minmod, include/Differ.hpp:33-43: R > 0 ? min(R, 1) : 0
-    return (R > P(0)) ? ((P(1) < R) ? P(1) : R) : P(0);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+__device__ __forceinline__ double rsqrt_approx(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+// 1/x within an ulp
+__device__ __forceinline__ double rcp_1ulp(double x)
+{
+    const double y = rcp_approx(x), e = __fma_rn(-x, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+// a/b from r = rcp_1ulp(b)
+__device__ __forceinline__ double div_by(double a, double b, double r)
+{
+    const double q = __dmul_rn(a, r);
+    return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+__device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, rcp_1ulp(b)); }
+__device__ __forceinline__ double rcp_rn(double x)
+{
+    const double y = rcp_1ulp(x);
+    return __fma_rn(__fma_rn(-x, y, 1.0), y, y);
+}
+// sqrt(x), x in the normal range or zero
+__device__ __forceinline__ double sqrt_rn(double x)
+{
+    const double y0 = rsqrt_approx(x);
+    const double e = __fma_rn(-__dmul_rn(x, y0), y0, 1.0);
+    const double y = __fma_rn(__dmul_rn(y0, e), __fma_rn(e, 0.375, 0.5), y0);
+    const double g = __dmul_rn(x, y);
+    return x == 0.0 ? x : __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
 }
 
 // Third-order WENO (Jiang and Shu, J. Comput. Phys. 126, 1996; new -- the
@@ -43,7 +82,7 @@ __device__ __forceinline__ double weno3(double far, double ctr, double oth)
     double q0 = __dadd_rn(1e-6, __dmul_rn(A0, A0)), q1 = __dadd_rn(1e-6, __dmul_rn(A1, A1));
     q0 = __dmul_rn(q0, q0);
     q1 = __dmul_rn(q1, q1);
-    const double w0 = __ddiv_rn(q1, __dadd_rn(q1, __dmul_rn(2.0, q0)));
+    const double w0 = div_rn(q1, __dadd_rn(q1, __dmul_rn(2.0, q0)));
     return __dadd_rn(ctr, __dmul_rn(0.5, __dadd_rn(A1, __dmul_rn(w0, __dsub_rn(A0, A1)))));
 }
 
@@ -59,32 +98,20 @@ __device__ __forceinline__ float weno3(float far, float ctr, float oth)
 // MUSCL_2 (limiter 0) face states, include/Differ.hpp:149-238 (MUSCL_1 when
 // DIFF == 0, :110-136; WENO above when DIFF == 2): the left state of the face
 // (i, i+1) from f(i-1), f(i), f(i+1), the right state from f(i), f(i+1),
-// f(i+2).
+// f(i+2).  FP32; the FP64 states are up_state below.
 template <class P, int DIFF>
 __device__ __forceinline__ P recon_left(P a, P b, P c)
 {
-    if (DIFF == EU3D_DIFF_MUSCL1) return b;
-    if (DIFF == EU3D_DIFF_WENO) return weno3(a, b, c);
-    const P kk = P(1.0) / P(3.0);
-    P A0 = b - a, A1 = c - b;
-    P Lr = A1 / (A0 + P(1e-12));
-    P L1 = minmod_lim(Lr), L2 = minmod_lim(P(1.0) / Lr);
-    return b + P(0.25) * ((P(1.0) - kk) * L1 + (P(1) + kk) * L2 * Lr) * A0;
+    return DIFF == EU3D_DIFF_WENO ? weno3(a, b, c) : b;
 }
 
 template <class P, int DIFF>
 __device__ __forceinline__ P recon_right(P b, P c, P d)
 {
-    if (DIFF == EU3D_DIFF_MUSCL1) return c;
-    if (DIFF == EU3D_DIFF_WENO) return weno3(d, c, b);
-    const P kk = P(1.0) / P(3.0);
-    P A1 = c - b, A2 = d - c;
-    P Rr = A1 / (A2 + P(1e-12));
-    P R1 = minmod_lim(Rr), R2 = minmod_lim(P(1.0) / Rr);
-    return c - P(0.25) * ((P(1.0) - kk) * R1 + (P(1) + kk) * R2 * Rr) * A2;
+    return DIFF == EU3D_DIFF_WENO ? weno3(d, c, b) : c;
 }
 
-// FP32 path: the same limited states without divisions.  With the minmod
+// MUSCL_2 without divisions.  With the minmod
 // limiter and kappa = 1/3, the reconstruction reduces to
 //     left  = f_i   + 0.5 * (L >= 1 ? A0 : L A0),  L = A1 / (A0 + 1e-12) > 0, else f_i
 //     right = f_i+1 - 0.5 * (R >= 1 ? A2 : R A2),  R = A1 / (A2 + 1e-12) > 0, else f_i+1
@@ -105,10 +132,6 @@ __device__ __forceinline__ float recon_right<float, EU3D_DIFF_MUSCL2>(float b, f
     const float r = __fmaf_rn(-0.5f, fabsf(A1) >= fabsf(e) ? A2 : A1, c);
     return __fmul_rn(A1, e) > 0.f ? r : c;
 }
-
-// a / b: IEEE in FP64 (parity path), the fast approximate form in FP32
-__device__ __forceinline__ double pdiv(double a, double b) { return a / b; }
-__device__ __forceinline__ float pdiv(float a, float b) { return __fdividef(a, b); }
 
 // the hardware's approximate reciprocal square root and reciprocal (PTX
 // rsqrt.approx / rcp.approx, subnormals flushed: the FP32 flux never meets
@@ -267,71 +290,131 @@ struct StridedSrc {
 };
 
 // Face flux between cells a and a+1 (cells a-1 .. a+2 along the direction,
-// element stride st, qc the index of cell a-1 of field 0).  FP64: the
-// reference's reconstruction with divisions; FP32: face_flux_src.
-template <class P, int DIR, int DIFF, bool LDG = true>
-__device__ __forceinline__ void face_flux_up(const P *__restrict__ qc, int fs, int st, bool zspec, P out[NV])
+// element stride st, qc the index of cell a-1 of field 0), FP32.
+template <int DIR, int DIFF, bool LDG = true>
+__device__ __forceinline__ void face_flux_up(const float *__restrict__ qc, int fs, int st, bool zspec, float out[NV])
 {
-    if constexpr (sizeof(P) == 4) {
-        face_flux_src<DIR, DIFF>(StridedSrc<LDG>{qc, fs, st}, zspec, out);
-        return;
-    } else {
-    // qc points at cell a-1 of field 0; field f of cell a-1+n is qc[f * fs + n * st]
-    auto ld = [&](int f, int n) -> P { return LDG ? __ldg(qc + f * fs + n * st) : qc[f * fs + n * st]; };
-    auto both = [&](int f, P &L, P &R) {
-        const P v0 = ld(f, 0), v1 = ld(f, 1), v2 = ld(f, 2), v3 = ld(f, 3);
-        L = recon_left<P, DIFF>(v0, v1, v2);
-        R = recon_right<P, DIFF>(v1, v2, v3);
+    face_flux_src<DIR, DIFF>(StridedSrc<LDG>{qc, fs, st}, zspec, out);
+}
+
+// ---- FP64 faces ----------------------------------------------------------
+// The reference forms each limited state with two divisions (Lr = A1 / (A0 +
+// 1e-12) and 1 / Lr) and each face's sound speeds and Mach numbers with more
+// of them and two square roots; compiled as they stand they made a cell 16 000
+// instructions, most in the divisions' out-of-line paths and the branches
+// around them.  The faces below give the same bits from straight-line code:
+// div_rn and sqrt_rn round as the IEEE operations do, and the limiter's cases
+// are selected,
+//     0 < Lr < 1: minmod(Lr) = Lr, minmod(1 / Lr) = 1;
+//     Lr >= 1:    minmod(Lr) = 1,  minmod(1 / Lr) = 1 / Lr;
+//     Lr <= 0:    both 0 (a NaN Lr gives a NaN state, as 0 * NaN does there).
+// Bit for bit matters: the adaptive chemistry behind a detonation doubles a
+// difference of the last bit in every step.  The two quarters of the kappa =
+// 1/3 weights (exact scalings) save the final product by 0.25.
+__device__ __forceinline__ double muscl2_weight(double A0, double A1, double seps)
+{
+    const double kk = 1.0 / 3.0;
+    const double c1 = 0.25 * (1.0 - kk), c2 = 0.25 * (1.0 + kk);
+    const double Lr = div_rn(A1, A0 + seps);
+    // comparisons on the high word (the FP64 pipe is the busy one): negative
+    // numbers count as below 1, a NaN's word is positive and above it
+    const int hi = __double2hiint(Lr);
+    const bool lt = hi < 0x3ff00000;
+    const double L1 = lt ? Lr : 1.0, L2 = lt ? 1.0 : rcp_rn(Lr);
+    const double w = __fma_rn(c1, L1, __dmul_rn(__dmul_rn(c2, L2), Lr));
+    return hi < 0 ? 0.0 : w;
+}
+
+// The state of cell ctr at the face towards oth: seps = 1e-12 for a left state
+// (far, ctr, oth = cells a-1, a, a+1), -1e-12 for a right one (a+2, a+1, a),
+// whose differences are the reference's with both signs turned.
+template <int DIFF>
+__device__ __forceinline__ double up_state(double far, double ctr, double oth, double seps)
+{
+    if (DIFF == EU3D_DIFF_MUSCL1) return ctr;
+    if (DIFF == EU3D_DIFF_WENO) return weno3(far, ctr, oth);
+    const double A0 = ctr - far;
+    return __fma_rn(muscl2_weight(A0, oth - ctr, seps), A0, ctr);
+}
+
+// One column of four cells a-1 .. a+2 for a face of k_flux64: byte offsets
+// from a field's first element, the same for every field.  The field bases
+// are uniform over the block, so a load needs no per-thread address
+// arithmetic beyond these offsets.
+struct FaceOff {
+    uint32_t o0, o1, o2, o3;
+};
+
+// the 16 fields' first elements, passed by value so that they sit in the
+// kernel's constant bank
+struct FieldBase {
+    const char *p[NPRIM];
+    __device__ __forceinline__ double ld(int f, uint32_t o) const
+    {
+        return __ldg(reinterpret_cast<const double *>(p[f] + o));
+    }
+};
+
+// AUSM face flux (src/Flowfield.cpp:1395-1500) between the cells o1 and o2 of
+// the direction whose normal velocity is field fn and whose tangential ones
+// are ft and fs; only the upwind side of the passive fields is reconstructed.
+// out: species, normal, first and second tangential momentum, energy.  The
+// direction is a run-time argument so that the kernel holds one copy of this
+// code (three copies and their set-up overflowed the instruction cache).
+template <int DIFF>
+__device__ __forceinline__ void face_flux64(const FieldBase &q, const FaceOff &o, int fn, int ft, int fs, bool zspec,
+                                            double out[NV])
+{
+    auto both = [&](int f, double &Lv, double &Rv) {
+        const double v0 = q.ld(f, o.o0), v1 = q.ld(f, o.o1), v2 = q.ld(f, o.o2), v3 = q.ld(f, o.o3);
+        Lv = up_state<DIFF>(v0, v1, v2, 1e-12);
+        Rv = up_state<DIFF>(v3, v2, v1, -1e-12);
     };
-    constexpr int FN = DIR == 1 ? PU : DIR == 2 ? PV : PW;
-    P DL, DR, PL, PR, GL, GR, NL, NR;
+    double DL, DR, PL, PR, GL, GR, NL, NR;
     both(PD, DL, DR);
     both(PP, PL, PR);
     both(PG, GL, GR);
-    both(FN, NL, NR);
-    const P CL = sqrt(pdiv(GL * PL, DL));
-    const P CR = sqrt(pdiv(GR * PR, DR));
-    const P CI = P(0.5) * (CL + CR);
-    const P MaL = pdiv(NL, CI), MaR = pdiv(NR, CI);
-    P B1, G1, B2, G2;
-    if (fabs(MaL) < P(1.0)) {
-        P mp = MaL + P(1.0), m2 = MaL * MaL - P(1.0);
-        B1 = P(0.25) * (mp * mp) + P(0.125) * (m2 * m2);
-        G1 = P(0.25) * (mp * mp) * (P(2.0) - MaL) + P(3.0) / P(16.0) * MaL * (m2 * m2);
-    } else {
-        B1 = P(0.5) * (MaL + fabs(MaL));
-        G1 = pdiv(B1, MaL);
+    both(fn, NL, NR);
+    const double CL = sqrt_rn(div_rn(GL * PL, DL));
+    const double CR = sqrt_rn(div_rn(GR * PR, DR));
+    const double CI = 0.5 * (CL + CR);
+    const double rCI = rcp_1ulp(CI);
+    const double MaL = div_by(NL, CI, rCI), MaR = div_by(NR, CI, rCI);
+    double B1, G1, B2, G2;
+    {
+        const double mp = MaL + 1.0, m2 = MaL * MaL - 1.0;
+        const double b = 0.25 * (mp * mp) + 0.125 * (m2 * m2);
+        const double g = 0.25 * (mp * mp) * (2.0 - MaL) + 3.0 / 16.0 * MaL * (m2 * m2);
+        const bool sub = fabs(MaL) < 1.0;
+        B1 = sub ? b : 0.5 * (MaL + fabs(MaL));
+        G1 = sub ? g : (MaL > 0.0 ? 1.0 : 0.0);  // (B1 / MaL exactly)
     }
-    if (fabs(MaR) < P(1.0)) {
-        P mm = MaR - P(1.0), m2 = MaR * MaR - P(1.0);
-        B2 = P(-0.25) * (mm * mm) - P(0.125) * (m2 * m2);
-        G2 = P(0.25) * (mm * mm) * (P(2.0) + MaR) - P(3.0) / P(16.0) * MaR * (m2 * m2);
-    } else {
-        B2 = P(0.5) * (MaR - fabs(MaR));
-        G2 = pdiv(B2, MaR);
+    {
+        const double mm = MaR - 1.0, m2 = MaR * MaR - 1.0;
+        const double b = -0.25 * (mm * mm) - 0.125 * (m2 * m2);
+        const double g = 0.25 * (mm * mm) * (2.0 + MaR) - 3.0 / 16.0 * MaR * (m2 * m2);
+        const bool sub = fabs(MaR) < 1.0;
+        B2 = sub ? b : 0.5 * (MaR - fabs(MaR));
+        G2 = sub ? g : (MaR < 0.0 ? 1.0 : 0.0);
     }
-    const P VI = (B1 + B2) * CI;
-    const bool left = VI >= P(0.0);
-    // upwind-side reconstruction of one field
-    auto up = [&](int f) -> P {
-        return left ? recon_left<P, DIFF>(ld(f, 0), ld(f, 1), ld(f, 2)) : recon_right<P, DIFF>(ld(f, 1), ld(f, 2), ld(f, 3));
-    };
-    const P Ds = left ? DL : DR;
-    const P Us = DIR == 1 ? (left ? NL : NR) : up(PU);
-    const P Vs = DIR == 2 ? (left ? NL : NR) : up(PV);
-    const P Ws = DIR == 3 ? (left ? NL : NR) : up(PW);
-    const P Hs = up(PH);
-    const P VD = VI * Ds;
+    const double VI = (B1 + B2) * CI;
+    const bool left = VI >= 0.0;
+    const uint32_t of = left ? o.o0 : o.o3, oc = left ? o.o1 : o.o2, oo = left ? o.o2 : o.o1;
+    const double seps = left ? 1e-12 : -1e-12;
+    auto up = [&](int f) -> double { return up_state<DIFF>(q.ld(f, of), q.ld(f, oc), q.ld(f, oo), seps); };
+    const double Ds = left ? DL : DR, Ns = left ? NL : NR;
+    const double Ts = up(ft), Ss = up(fs), Hs = up(PH);
+    const double VD = VI * Ds;
+    out[NS] = VD * Ns + G1 * PL + G2 * PR;
+    out[NS + 1] = VD * Ts;
+    out[NS + 2] = VD * Ss;
+    // u^2 + v^2 + w^2 and the energy sum in the operation order that a
+    // compiled face of fixed direction and scheme has
+    const double p2 = fn == PW ? Ss : Ns, r2 = fn == PW ? Ns : Ss;
+    const double q2 = __fma_rn(r2, r2, __fma_rn(p2, p2, __dmul_rn(Ts, Ts))), hd = 0.5 * Ds;
+    out[NS + 3] = VI * (DIFF == EU3D_DIFF_WENO ? __fma_rn(hd, q2, __dmul_rn(Ds, Hs)) : __fma_rn(Ds, Hs, __dmul_rn(hd, q2)));
 #pragma unroll
-    for (int s = 0; s < NS; s++) out[s] = zspec ? P(0) * VD : VD * up(PY + s);
-    out[NS] = VD * Us;
-    out[NS + 1] = VD * Vs;
-    out[NS + 2] = VD * Ws;
-    if (DIR == 1) out[NS] = VD * Us + G1 * PL + G2 * PR;
-    if (DIR == 2) out[NS + 1] = VD * Vs + G1 * PL + G2 * PR;
-    if (DIR == 3) out[NS + 2] = VD * Ws + G1 * PL + G2 * PR;
-    out[NS + 3] = VI * (Ds * Hs + P(0.5) * Ds * (Us * Us + Vs * Vs + Ws * Ws));
-    }
+    for (int s = 0; s < NS; s++) out[s] = zspec ? 0.0 * VD : VD * up(PY + s);
 }
 
 // Wedge immersed boundary as the flux kernels see it: a tile none of whose
@@ -347,43 +430,146 @@ struct FluxSolid {
 };
 
 constexpr int FT_X = 32;
-// tile height: 8 rows for FP32 primitives, 4 for FP64; face fluxes live in
-// dynamic shared memory (two buffers of x and y faces)
-template <class P>
-struct FluxTile {
-    static constexpr int TY = sizeof(P) == 8 ? 4 : 8;
-    static constexpr int FX = TY * (FT_X + 1) * NV;  // elements of one x-face buffer
-    static constexpr int FY = (TY + 1) * FT_X * NV;  // elements of one y-face buffer
-    static constexpr size_t SMEM = sizeof(P) * 2 * (FX + FY);
+
+// FP64 flux + residual kernel.  A block owns a 32 x TY tile of x-y columns and
+// walks `kz` z planes.  At each plane every thread of the TY cell warps
+// evaluates the lower y face, the left x face and the upper z face of its
+// cell, in a loop over the three directions; one extra warp adds the tile's
+// last y-face row and then the last x face of each row.  Lanes past a ragged
+// edge repeat clamped cells and store nothing, so no lane leaves the code.
+// x and y fluxes go through shared memory, the z face below a cell is the face
+// above the previous plane's cell.  The residual is formed in the reference's
+// order ((-dt/dx dF - dt/dy dG) - dt/dz dQ).
+// Cells are read through L1: the four planes a z face spans and the tile's
+// halo are re-read from L1 and L2, whose bandwidth is not the bound (232 B a
+// cell of HBM traffic).  What bounds it is the FP64 pipe together with issue
+// and latency: 3780 warp instructions a cell, 1710 of them FP64 (two cycles
+// each), at 16 warps an SM (128 registers).  160^3: 0.75 ms a launch; 6.4 ms
+// with the compiler's quotients (16 000 instructions a cell, an FP64 pipe 12 %
+// busy behind branches, barriers and instruction fetches).  Left out, measured
+// on a cheaper form of the limiter: three inlined copies of the face (0.77 ms
+// against 0.62: instruction cache), 96 registers and 20 warps (0.77), an L2
+// prefetch of plane k + 3 (0.58 against 0.56), per-load address products
+// instead of field bases in the constant bank (0.62 against 0.56).
+template <int TY>
+struct Flux64 {
+    static constexpr int THREADS = FT_X * (TY + 1);
+    static constexpr int FY = (TY + 1) * NV * FT_X;   // y-face fluxes
+    static constexpr int FX = TY * NV * (FT_X + 1);   // x-face fluxes
+    static constexpr size_t SMEM = sizeof(double) * (FY + FX + 1);
 };
 
-// Tiled flux + residual kernel.  A block owns a 32 x TY tile of x-y columns
-// and walks `kz` z planes.  At each plane every x face and y face of the tile
-// is computed once (by one thread) into shared memory, every z face once in
-// registers (the face below a cell is the face above the previous plane's
-// cell), and each thread then forms its cell's residual in the reference's
-// order ((-dt/dx dF - dt/dy dG) - dt/dz dQ) in FP64.
-// A tile of 32 x TY cells has 33 x TY x faces and 32 x (TY + 1) y faces: the
-// block carries two extra warps, one for the last y-face row (ty == TY) and
-// one for the last x face of each row (ty == TY + 1), so that every warp
-// evaluates at most one face of each direction per plane.
-template <class P>
-constexpr int flux_threads()
+template <int DIFF, bool SQ, int TY, int NB>
+__global__ void __launch_bounds__(Flux64<TY>::THREADS, NB) k_flux64(
+    Layout L, const __grid_constant__ FieldBase qf, const double *__restrict__ xn, const double *__restrict__ yn,
+    const double *__restrict__ zn, const double *__restrict__ dtp, double *__restrict__ rhs, int kz, FluxSolid wedge)
 {
-    return FT_X * (FluxTile<P>::TY + 2);
+    extern __shared__ __align__(16) double f64_smem[];
+    double *const fy = f64_smem, *const fx = fy + Flux64<TY>::FY, *const czb = fx + Flux64<TY>::FX;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int i0 = L.bc + blockIdx.x * FT_X, j0 = L.bc + blockIdx.y * TY;
+    const int kb = L.bc + blockIdx.z * kz;
+    const int ke = min(kb + kz, L.nk + L.bc);
+    const int i = i0 + tx, j = j0 + ty;
+    const int ilast = L.ni + L.bc - 1, jlast = L.nj + L.bc - 1;
+    const bool cellw = ty < TY;  // warps that own cells (the other one only adds faces)
+    const bool act = cellw && i <= ilast && j <= jlast;
+    if (!__syncthreads_or(act && !wedge.solid(xn[i], yn[j]))) return;  // an all-solid tile
+    const uint32_t sx = 8u, sy = 8u * (uint32_t)L.px, sz = sy * (uint32_t)L.NJ;
+    const double dt = *dtp;
+    // the cell whose upper z face this thread owns, the right cell of its x
+    // face and the upper cell of its y face, clamped into the array (ilast + 1
+    // and jlast + 1 are ghosts)
+    const int ic = min(i, ilast), jc = min(j, jlast);
+    const int xrow = cellw ? jc : min(j0 + min(tx, TY - 1), jlast);
+    const int ix = min(cellw ? i : i0 + FT_X, ilast + 1);
+    const bool zs_cell = SQ && i >= L.ni, zs_x = SQ && ix - 1 >= L.ni;
+    uint32_t oz = (uint32_t)L.at(ic, jc, kb) * 8u - sz;
+    uint32_t ox = (uint32_t)L.at(ix, xrow, kb) * 8u;
+    uint32_t oy = (uint32_t)L.at(ic, min(j, jlast + 1), kb) * 8u;
+    double *const sfy = fy + ty * NV * FT_X + tx;
+    double *const sfx = fx + (cellw ? ty * NV * (FT_X + 1) + tx : min(tx, TY - 1) * NV * (FT_X + 1) + FT_X);
+    double qb[NV], o[NV];
+    const double ax = act ? -dt / (xn[ic] - xn[ic - 1]) : 0.0;
+    const double by = act ? dt / (yn[jc] - yn[jc - 1]) : 0.0;
+    double *out = rhs + L.at(ic, jc, kb);
+    // the first pass forms only the z face below the first plane
+    for (int k = kb - 1; k < ke; k++) {
+        const bool first = k < kb;
+        if (!cellw && tx == 0 && !first) *czb = dt / (zn[k] - zn[k - 1]);
+#pragma unroll 1
+        for (int dir = first ? 2 : 0; dir < (cellw ? 3 : 2); dir++) {
+            const uint32_t st = dir == 0 ? sy : dir == 1 ? sx : sz;
+            const uint32_t c = dir == 0 ? oy : dir == 1 ? ox : oz + sz;
+            const int fn = dir == 0 ? PV : dir == 1 ? PU : PW;
+            const int ft = dir == 1 ? PV : PU, fs = dir == 2 ? PV : PW;
+            face_flux64<DIFF>(qf, FaceOff{c - 2 * st, c - st, c, c + st}, fn, ft, fs, dir == 1 ? zs_x : zs_cell, o);
+            if (dir == 2) break;
+            double *const d = dir == 0 ? sfy : sfx;
+            const int ld = dir == 0 ? FT_X : FT_X + 1;
+            // momenta to their places: y (V, U, W), x (U, V, W)
+            const int m0 = dir == 0 ? NS + 1 : NS, m1 = dir == 0 ? NS : NS + 1;
+#pragma unroll
+            for (int v = 0; v < NS; v++) d[v * ld] = o[v];
+            d[m0 * ld] = o[NS];
+            d[m1 * ld] = o[NS + 1];
+            d[(NS + 2) * ld] = o[NS + 2];
+            d[(NS + 3) * ld] = o[NS + 3];
+        }
+        // z momenta (W, U, V)
+        {
+            const double w = o[NS];
+            o[NS] = o[NS + 1];
+            o[NS + 1] = o[NS + 2];
+            o[NS + 2] = w;
+        }
+        if (!first) {
+            __syncthreads();
+            if (cellw) {
+                const double cz = *czb;
+#pragma unroll
+                for (int v = 0; v < NV; v++) {
+                    const double r = residual(ax, by, cz, sfx[v * (FT_X + 1) + 1], sfx[v * (FT_X + 1)],
+                                              sfy[(NV + v) * FT_X], sfy[v * FT_X], o[v], qb[v]);
+                    if (act) out[v * L.fs] = r;
+                }
+                out += sz / 8;
+            }
+            __syncthreads();
+            ox += sz;
+            oy += sz;
+        }
+        oz += sz;
+#pragma unroll
+        for (int v = 0; v < NV; v++) qb[v] = o[v];
+    }
 }
 
-template <class P, int DIFF>
-__global__ void __launch_bounds__(flux_threads<P>(), 2) k_flux_tile(
-    Layout L, const P *__restrict__ q, const double *__restrict__ xn, const double *__restrict__ yn,
-    const double *__restrict__ zn, const double *__restrict__ dtp, P *__restrict__ rhs, int species_quirk, int kz,
+// FP32 tiled kernel that reads the primitives through L1 (flux_stage 0), the
+// fallback of the staged kernels below.  A block owns a 32 x 8 tile of x-y
+// columns and walks `kz` z planes; every x and y face of the tile is computed
+// once into shared memory, every z face once in registers.  Two extra warps
+// take the last y-face row (ty == TY) and the last x face of each row
+// (ty == TY + 1), so that every warp evaluates at most one face of each
+// direction per plane.
+struct FluxTile {
+    static constexpr int TY = 8;
+    static constexpr int FX = TY * (FT_X + 1) * NV;  // elements of one x-face buffer
+    static constexpr int FY = (TY + 1) * FT_X * NV;  // elements of one y-face buffer
+    static constexpr size_t SMEM = sizeof(float) * 2 * (FX + FY);
+};
+
+template <int DIFF>
+__global__ void __launch_bounds__(FT_X *(FluxTile::TY + 2), 2) k_flux_tile(
+    Layout L, const float *__restrict__ q, const double *__restrict__ xn, const double *__restrict__ yn,
+    const double *__restrict__ zn, const double *__restrict__ dtp, float *__restrict__ rhs, int species_quirk, int kz,
     FluxSolid wedge)
 {
-    constexpr int TY = FluxTile<P>::TY;
+    constexpr int TY = FluxTile::TY;
     // two buffers: plane k+1 may fill one while slow threads still read plane k
     extern __shared__ __align__(16) unsigned char flux_smem[];
-    auto fx = reinterpret_cast<P(*)[TY][FT_X + 1][NV]>(flux_smem);
-    auto fy = reinterpret_cast<P(*)[TY + 1][FT_X][NV]>(flux_smem + sizeof(P) * 2 * FluxTile<P>::FX);
+    auto fx = reinterpret_cast<float(*)[TY][FT_X + 1][NV]>(flux_smem);
+    auto fy = reinterpret_cast<float(*)[TY + 1][FT_X][NV]>(flux_smem + sizeof(float) * 2 * FluxTile::FX);
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int i0 = L.bc + blockIdx.x * FT_X, j0 = L.bc + blockIdx.y * TY;
     const int kb = L.bc + blockIdx.z * kz;
@@ -396,10 +582,10 @@ __global__ void __launch_bounds__(flux_threads<P>(), 2) k_flux_tile(
     const int fs = (int)L.fs, sy = L.px, sz = L.px * L.NJ;
     const double dt = *dtp;
     const bool zs_cell = species_quirk && i >= L.ni;
-    P qb[NV], qa[NV];
-    const P ax = (P)(act ? -dt / (xn[i] - xn[i - 1]) : 0.0);
-    const P by = (P)(act ? dt / (yn[j] - yn[j - 1]) : 0.0);
-    if (act) face_flux_up<P, 3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
+    float qb[NV], qa[NV];
+    const float ax = (float)(act ? -dt / (xn[i] - xn[i - 1]) : 0.0);
+    const float by = (float)(act ? dt / (yn[j] - yn[j - 1]) : 0.0);
+    if (act) face_flux_up<3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
     for (int k = kb, it = 0; k < ke; k++, it ^= 1) {
         // x faces of row r: face f sits between a = i0+f-1 and a+1 and is
         // needed when a <= ilast; it reads cells a-1 .. a+2.  Faces 0..31 by
@@ -410,18 +596,18 @@ __global__ void __launch_bounds__(flux_threads<P>(), 2) k_flux_tile(
             const int jr = j0 + r;
             const int a = i0 + f - 1;
             if ((cellw || (ty == TY + 1 && tx < TY)) && jr <= jlast && a <= ilast)
-                face_flux_up<P, 1, DIFF>(q + L.at(a - 1, jr, k), fs, 1, species_quirk && a >= L.ni, fx[it][r][f]);
+                face_flux_up<1, DIFF>(q + L.at(a - 1, jr, k), fs, 1, species_quirk && a >= L.ni, fx[it][r][f]);
         }
         // y faces of column i: face g sits between b = j0+g-1 and b+1;
         // faces 0..TY-1 by the cell warps, face TY by warp TY
         if (ty <= TY && i <= ilast) {
             const int b = j0 + ty - 1;
-            if (b <= jlast) face_flux_up<P, 2, DIFF>(q + L.at(i, b - 1, k), fs, sy, species_quirk && i >= L.ni, fy[it][ty][tx]);
+            if (b <= jlast) face_flux_up<2, DIFF>(q + L.at(i, b - 1, k), fs, sy, species_quirk && i >= L.ni, fy[it][ty][tx]);
         }
-        if (act) face_flux_up<P, 3, DIFF>(q + L.at(i, j, k) - sz, fs, sz, zs_cell, qa);
+        if (act) face_flux_up<3, DIFF>(q + L.at(i, j, k) - sz, fs, sz, zs_cell, qa);
         __syncthreads();
         if (act) {
-            const P cz = (P)(dt / (zn[k] - zn[k - 1]));
+            const float cz = (float)(dt / (zn[k] - zn[k - 1]));
             const long long c = L.at(i, j, k);
 #pragma unroll
             for (int v = 0; v < NV; v++) {
@@ -474,7 +660,7 @@ __global__ void __launch_bounds__(FT_X *(FS_TY + 2), 2) k_flux_stage(
     float qb[NV], qa[NV];
     const float ax = (float)(act ? -dt / (xn[i] - xn[i - 1]) : 0.0);
     const float by = (float)(act ? dt / (yn[j] - yn[j - 1]) : 0.0);
-    if (act) face_flux_up<float, 3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
+    if (act) face_flux_up<3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
     for (int k = kb; k < ke; k++) {
         // stage cells x in [i0 - 2, i0 + 34), y in [j0 - 2, j0 + TY + 2) of plane k
         // (indices past the array, never needed by a face, are clamped)
@@ -493,15 +679,15 @@ __global__ void __launch_bounds__(FT_X *(FS_TY + 2), 2) k_flux_stage(
             const int jr = j0 + r;
             const int a = i0 + f - 1;
             if ((cellw || (ty == TY + 1 && tx < TY)) && jr <= jlast && a <= ilast)
-                face_flux_up<float, 1, DIFF, false>(S + (r + 2) * HX + f, PL, 1, species_quirk && a >= L.ni, fx[r][f]);
+                face_flux_up<1, DIFF, false>(S + (r + 2) * HX + f, PL, 1, species_quirk && a >= L.ni, fx[r][f]);
         }
         // y face g of column i: between b = j0+g-1 and b+1, staged rows g .. g+3
         if (ty <= TY && i <= ilast) {
             const int b = j0 + ty - 1;
             if (b <= jlast)
-                face_flux_up<float, 2, DIFF, false>(S + ty * HX + tx + 2, PL, HX, species_quirk && i >= L.ni, fy[ty][tx]);
+                face_flux_up<2, DIFF, false>(S + ty * HX + tx + 2, PL, HX, species_quirk && i >= L.ni, fy[ty][tx]);
         }
-        if (act) face_flux_up<float, 3, DIFF>(q + L.at(i, j, k) - sz, fs, sz, zs_cell, qa);
+        if (act) face_flux_up<3, DIFF>(q + L.at(i, j, k) - sz, fs, sz, zs_cell, qa);
         __syncthreads();
         if (act) {
             const float cz = (float)(dt / (zn[k] - zn[k - 1]));
@@ -768,7 +954,7 @@ __global__ void __launch_bounds__(FT_X *(FR_TY + 2), 2) k_flux_ring(
     // plane kb - 1 into the thread's slot
     float *slot = core + (cellw ? tid : 0);
     if (act) {
-        face_flux_up<float, 3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
+        face_flux_up<3, DIFF>(q + L.at(i, j, kb) - 2 * (long long)sz, fs, sz, zs_cell, qb);
         const float *g = q + L.at(i, j, kb) - sz;
 #pragma unroll
         for (int f = 0; f < NPRIM; f++) slot[f * FR_CS] = __ldg(g + (long long)f * fs);
