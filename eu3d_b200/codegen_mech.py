@@ -111,7 +111,7 @@ def gen(mech) -> str:
     w("")
 
     # one reaction's rate block
-    def reaction(r, rtb_expr):
+    def reaction(r, rtb_expr, fast):
         xr = float(np.sum(sb[:, r] - sf[:, r]))
         b = float(mech.bf[r])
         if b == 0.0:
@@ -129,7 +129,8 @@ def gen(mech) -> str:
         if mech.eaf[r] == 0.0:
             o.append(f"        const double kf = {lit(mech.af[r])} * {powt};")
         else:
-            o.append(f"        const double kf = {lit(mech.af[r])} * {powt} * exp(-{lit(mech.eaf[r])} / (RU_CAL * p.T));")
+            arg = f"div_by(-{lit(mech.eaf[r])}, rut, irut)" if fast else f"-{lit(mech.eaf[r])} / (RU_CAL * p.T)"
+            o.append(f"        const double kf = {lit(mech.af[r])} * {powt} * exp({arg});")
         terms = []
         for s in range(NS):
             nu = sb[s, r] - sf[s, r]
@@ -162,8 +163,9 @@ def gen(mech) -> str:
             kc = f"kp * (R_GAS * p.T)"
         else:
             kc = f"kp * pow(R_GAS * p.T, {lit(-xr)})"
-        o.append(f"        const double kp = exp(-dg / (R_GAS * p.T)) * {lit(p0)};")
-        o.append(f"        const double kb = kf / ({kc});")
+        arg = "div_by(-dg, rgt, irgt)" if fast else "-dg / (R_GAS * p.T)"
+        o.append(f"        const double kp = exp({arg}) * {lit(p0)};")
+        o.append(f"        const double kb = {f'div_rn(kf, {kc})' if fast else f'kf / ({kc})'};")
         if has_tb:
             o.append(f"        double tb = {' + '.join(tbt)};")
         else:
@@ -173,7 +175,11 @@ def gen(mech) -> str:
         return o, has_tb
 
     # IMEX: Diagonalized (R_TB defaults to 1)
-    w("// Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s)")
+    w("// Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s).  For T in")
+    w("// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in")
+    w("// the normal range (common.cuh's div_rn); the caller takes the table-driven")
+    w("// form elsewhere.")
+    w("constexpr double FAST_T_LO = 150.0, FAST_T_HI = 1e4;")
     w("__device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[NS], const double Mc[NS],")
     w("                                                  const double Di[NS], const double PT[NS], double CMS[NS],")
     w("                                                  double MD[NS])")
@@ -190,14 +196,15 @@ def gen(mech) -> str:
     w("#pragma unroll")
     w("    for (int s = 0; s < NS; s++) {")
     w("        sDi[s] = fabs(Di[s]) < 0x1p-1022 ? 0x1p+64 : 1.0;")
-    w("        iDi[s] = Di[s] == 0.0 ? 0.0 : 1.0 / (Di[s] * sDi[s]);")
+    w("        iDi[s] = Di[s] == 0.0 ? 0.0 : rcp_rn(Di[s] * sDi[s]);")
     w("    }")
-    w("    const double tdep = 1.0 / (RU_CAL * (p.T * p.T));")
+    w("    const double rut = RU_CAL * p.T, irut = rcp_1ulp(rut), rgt = R_GAS * p.T, irgt = rcp_1ulp(rgt);")
+    w("    const double tdep = rcp_rn(RU_CAL * (p.T * p.T));")
     w("#pragma unroll")
     w("    for (int s = 0; s < NS; s++) { Wi[s] = 0.0; MD[s] = 0.0; }")
     for r in range(NR):
         w("    {")
-        blk, has_tb = reaction(r, "if (tb == 0.0) tb = 1.0;")
+        blk, has_tb = reaction(r, "if (tb == 0.0) tb = 1.0;", True)
         L.extend(blk)
         wt = []
         if mech.bf[r] != 0.0:
@@ -241,7 +248,7 @@ def gen(mech) -> str:
     w("    for (int s = 0; s < NS; s++) { Wi[s] = 0.0; Pv[s] = 0.0; Qv[s] = 0.0; }")
     for r in range(NR):
         w("    {")
-        blk, has_tb = reaction(r, "if (rtb_mode == 0) { if (tb == 0.0) tb = 1.0; } else if (rtb_mode == 2) { tb = 0.0; }")
+        blk, has_tb = reaction(r, "if (rtb_mode == 0) { if (tb == 0.0) tb = 1.0; } else if (rtb_mode == 2) { tb = 0.0; }", False)
         L.extend(blk)
         for s in range(NS):
             nu = sb[s, r] - sf[s, r]

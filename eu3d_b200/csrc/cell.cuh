@@ -47,7 +47,7 @@ __device__ __forceinline__ void decode(const double cs[NV], double T0, double Eo
 #pragma unroll
     for (int s = 0; s < NS; s++) D += cs[s];
     // one reciprocal of the density serves every quotient (within an ulp of dividing)
-    const double iD = 1.0 / D;
+    const double iD = rcp_rn(D);
     double yr[NS], sYR = 0.0, sdiv = 0.0;
 #pragma unroll
     for (int s = 0; s < NS; s++) {
@@ -75,7 +75,7 @@ __device__ __forceinline__ void decode(const double cs[NV], double T0, double Eo
         const double scp = A[0] * p.tm2 + A[1] * p.tm1 + A[2] + A[3] * p.T + A[4] * p.t2 + A[5] * p.t3 + A[6] * p.t4;
         const double t1 = (sh - Et * 1e-3) - sYR * Tp;
         const double t2 = scp - sYR;
-        Tn = Tp - t1 / t2;
+        Tn = Tp - div_rn(t1, t2);
         if (fabs(Tn - Tp) < 1e-6) break;
         count++;
     }
@@ -83,12 +83,12 @@ __device__ __forceinline__ void decode(const double cs[NV], double T0, double Eo
     const TPow p = tpow(Tn, q);
     if (p.hi != cur) mix_coeffs(yr, p.hi, p.rb, A);
     const double scp = A[0] * p.tm2 + A[1] * p.tm1 + A[2] + A[3] * p.T + A[4] * p.t2 + A[5] * p.t3 + A[6] * p.t4;
-    const double Wav = 1.0 / sdiv;
-    o.Rgas = R_GAS * 1000 / Wav;
+    const double Wav = rcp_rn(sdiv);
+    o.Rgas = div_rn(R_GAS * 1000, Wav);
     o.P = Tn * D * o.Rgas;
-    o.H = o.P / D + Enew;
+    o.H = div_by(o.P, D, iD) + Enew;
     o.Cp = scp * 1000;
-    o.G = o.Cp / (o.Cp - R_GAS * sdiv * 1000);
+    o.G = div_rn(o.Cp, o.Cp - R_GAS * sdiv * 1000);
     o.D = D;
     o.U = U;
     o.V = V;
@@ -315,18 +315,31 @@ __device__ __forceinline__ void warp_sum(unsigned long long *ctr, unsigned long 
 // source CMS (kg/m^3/s) and diagonal MD of the partial densities.
 // tcouple = false drops the temperature coupling of the Jacobian (PT = 0),
 // leaving its composition part (the adaptive integrator below).
-template <bool SPEC>
-__device__ __forceinline__ void imex_source(const double cs[NV], double T, unsigned qk, double CMS[NS], double MD[NS],
-                                            bool tcouple = true)
+//
+// Two forms.  The compiled-in mechanism between FAST_T_LO and FAST_T_HI takes
+// the specialised rates with common.cuh's straight-line quotients: the same
+// bits as the compiler's divisions, of which a cell has some 120, in two
+// thirds of the instructions and without their branches, which kept the
+// scheduler from overlapping the 33 exponentials.  1.3 M cells: IMEX 0.85 ->
+// 0.40 ms (cold flow) and 0.69 -> 0.41 (hot), the adaptive chemistry on hot
+// gas 27.9 -> 16.5 ms.  Every other cell (and every other mechanism) takes the
+// table-driven form: below 150 K and above 1e4 K an equilibrium constant may
+// leave the range in which the quotients round as IEEE's.
+template <bool FAST>
+__device__ __forceinline__ void imex_source_t(const double cs[NV], double T, unsigned qk, double CMS[NS], double MD[NS],
+                                              bool tcouple)
 {
+    auto quot = [](double a, double b, double r) { return FAST ? div_by(a, b, r) : a / b; };
+    auto recip = [](double b) { return FAST ? rcp_1ulp(b) : 0.0; };
     // state of the previous decode, recomputed from the stored CS and T
     double D = 0.0;
 #pragma unroll
     for (int s = 0; s < NS; s++) D += cs[s];
-    const double U = cs[NS] / D, V = cs[NS + 1] / D, W = cs[NS + 2] / D;
+    const double rD = recip(D);
+    const double U = quot(cs[NS], D, rD), V = quot(cs[NS + 1], D, rD), W = quot(cs[NS + 2], D, rD);
     const TPow p = tpow(T, qk);
     double hr[NS], sr[NS], cpr[NS];
-    if (SPEC) {
+    if (FAST) {
         h2ja919::thermo_spec(p, hr, sr, cpr);
     } else {
 #pragma unroll
@@ -339,26 +352,67 @@ __device__ __forceinline__ void imex_source(const double cs[NV], double T, unsig
     double sdiv = 0.0, scp = 0.0, Mc[NS], Di[NS], PT[NS], G[NS];
 #pragma unroll
     for (int s = 0; s < NS; s++) {
-        const double Y = cs[s] / D;
-        sdiv += Y / cM.mw[s];
+        const double Y = quot(cs[s], D, rD);
+        sdiv += quot(Y, cM.mw[s], cM.imw[s]);
         scp += (cM.ri[s] * cpr[s]) * Y;
     }
-    const double Rgas = R_GAS * 1000 / (1.0 / sdiv);
+    const double Rgas = FAST ? div_rn(R_GAS * 1000, rcp_rn(sdiv)) : R_GAS * 1000 / (1.0 / sdiv);
     const double CV = scp * 1000 - Rgas;
     const double ke = 0.5 * (U * U + V * V + W * W);
+    const double CVD = CV * D, rCVD = recip(CVD);
     // GetPartial_T, src/Flowfield.cpp:1578-1595; Gibbs energies for the rates
 #pragma unroll
     for (int s = 0; s < NS; s++) {
         const double hs = (qk & EU3D_Q_PARTIAL_T_UNITS) ? cM.ri[s] * hr[s] : (cM.ri[s] * hr[s]) * 1e3;
-        PT[s] = tcouple ? (ke - hs + cM.ri[s] * 1e3 * T) / (CV * D) : 0.0;
+        PT[s] = tcouple ? quot(ke - hs + cM.ri[s] * 1e3 * T, CVD, rCVD) : 0.0;
         G[s] = R_GAS * hr[s] - (R_GAS * sr[s]) * T;
         Di[s] = cs[s] * 1e-3;
-        Mc[s] = (cs[s] / cM.mw[s] * 1000) * 1e-6;
+        Mc[s] = (quot(cs[s], cM.mw[s], cM.imw[s]) * 1000) * 1e-6;
     }
-    if (SPEC)
+    if (FAST)
         h2ja919::diagonalized_spec(p, G, Mc, Di, PT, CMS, MD);
     else
         diagonalized(p, G, Mc, Di, PT, CMS, MD);
+}
+
+// where the specialised form holds: every rate constant and quotient in the
+// normal range
+__device__ __forceinline__ bool imex_fast_ok(double T, double D)
+{
+    return T >= h2ja919::FAST_T_LO && T <= h2ja919::FAST_T_HI && D >= 1e-30 && D <= 1e30;
+}
+
+// the table-driven form out of line for the rare cells outside the fast range
+static __device__ __noinline__ void imex_source_rare(const double *cs, double T, unsigned qk, double *CMS, double *MD,
+                                                     bool tcouple)
+{
+    imex_source_t<false>(cs, T, qk, CMS, MD, tcouple);
+}
+
+template <bool SPEC>
+__device__ __forceinline__ void imex_source(const double cs[NV], double T, unsigned qk, double CMS[NS], double MD[NS],
+                                            bool tcouple = true)
+{
+    if (!SPEC) {
+        imex_source_t<false>(cs, T, qk, CMS, MD, tcouple);
+        return;
+    }
+    double D = 0.0;
+#pragma unroll
+    for (int s = 0; s < NS; s++) D += cs[s];
+    if (imex_fast_ok(T, D)) {
+        imex_source_t<true>(cs, T, qk, CMS, MD, tcouple);
+    } else {
+        double c[NV], cm[NS], md[NS];
+#pragma unroll
+        for (int v = 0; v < NV; v++) c[v] = cs[v];
+        imex_source_rare(c, T, qk, cm, md, tcouple);
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            CMS[s] = cm[s];
+            MD[s] = md[s];
+        }
+    }
 }
 
 // FP64 adaptive closed-reactor chemistry (new; the reference's one-step IMEX
@@ -394,15 +448,16 @@ __device__ __forceinline__ void adapt_substep(double cs[NV], double &T, double E
 #pragma unroll
     for (int s = 0; s < NS; s++) {
         const double w = fabs(CMS[s]);
-        if (w > 0.0) h = fmin(h, cfg.rel * (cs[s] + 1e-9 * D) / w);
-        if (MD[s] > 0.0) h = fmin(h, cfg.amp / MD[s]);
+        // (a quotient past the largest number comes out as NaN, which fmin drops)
+        if (w > 0.0) h = fmin(h, div_rn(cfg.rel * (cs[s] + 1e-9 * D), w));
+        if (MD[s] > 0.0) h = fmin(h, div_rn(cfg.amp, MD[s]));
     }
     const double hc = h;
     h = fmin(fmax(h, hmin), trem);
     if (k == cfg.nmax - 1) h = trem;
     if (h > hc) forced = 1;
 #pragma unroll
-    for (int s = 0; s < NS; s++) cs[s] = fmax(cs[s] + h * CMS[s] / (1.0 - h * MD[s]), 0.0);
+    for (int s = 0; s < NS; s++) cs[s] = fmax(cs[s] + div_rn(h * CMS[s], 1.0 - h * MD[s]), 0.0);
     int cp = 0;
     decode(cs, T, Eold, qk, o, cp);
     capped_any |= cp;
@@ -604,6 +659,51 @@ __device__ __forceinline__ int adapt_split_step(const CellArgs &a, long long c, 
     return n;
 }
 
+// Flowfield::Update_IMEX, src/Flowfield.cpp:1219-1228
+template <class P>
+__device__ __forceinline__ void imex_update(const CellArgs &a, long long c, double cs[NV], const double CMS[NS],
+                                            const double MD[NS])
+{
+    const double dt = a.scal[0];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+        double r = rhs_at<P>(a, v * a.L.fs + c);
+        if (v < NS) {
+            r = r + CMS[v] * dt;
+            cs[v] = cs[v] + div_rn(r, 1.0 - dt * MD[v]);
+        } else {
+            cs[v] = cs[v] + r;
+        }
+    }
+}
+
+// M_IMEX of one cell outside the specialised rates' range (divisions as the
+// compiler forms them)
+template <class P>
+__device__ __noinline__ void imex_cell_rare(const CellArgs *ap, P *q, long long c)
+{
+    const CellArgs &a = *ap;
+    const long long fs = a.L.fs;
+    const double dt = a.scal[0], T = a.T[c];
+    double cs[NV], CMS[NS], MD[NS];
+    load_cs(a.cs, fs, c, cs);
+    imex_source_t<false>(cs, T, a.quirks, CMS, MD, true);
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+        const double r = rhs_at<P>(a, v * fs + c);
+        cs[v] = v < NS ? cs[v] + (r + CMS[v] * dt) / (1.0 - dt * MD[v]) : cs[v] + r;
+    }
+    Decoded o;
+    int capped = 0;
+    decode(cs, T, (a.quirks & EU3D_Q_STALE_E) ? a.E[c] : 0.0, a.quirks, o, capped);
+    store_cs(a.cs, fs, c, cs);
+    a.T[c] = o.T;
+    a.E[c] = o.E;
+    store_prims<P>(o, q, fs, c);
+    if (capped) atomicAdd(&a.st->newton_capped, 1ull);
+    if (!(isfinite(o.D) && isfinite(o.T))) atomicAdd(&a.st->nonfinite, 1ull);
+}
+
 // One thread per interior cell.  MODE selects the reference sequence:
 //  M_DECODE  Update_after_CS
 //  M_ADV     Update_after_Adv (+ decode)
@@ -648,21 +748,25 @@ __device__ __forceinline__ void cell_body(const CellArgs &a, P *__restrict__ q, 
     int capped = 0, capped_any = 0;
 
     if (MODE == M_IMEX) {
-        double CMS[NS], MD[NS];
-        imex_source<SPEC>(cs, T, qk, CMS, MD);
-        // Flowfield::Update_IMEX, src/Flowfield.cpp:1219-1228
+        bool rare = false;
+        if (SPEC) {
+            double D = 0.0;
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-            double r = rhs_at<P>(a, v * fs + c);
-            if (v < NS) {
-                r = r + CMS[v] * dt;
-                cs[v] = cs[v] + r / (1.0 - dt * MD[v]);
-            } else {
-                cs[v] = cs[v] + r;
-            }
+            for (int s = 0; s < NS; s++) D += cs[s];
+            rare = !imex_fast_ok(T, D);
         }
+        double CMS[NS], MD[NS];
+        imex_source_t<SPEC>(cs, T, qk, CMS, MD, true);
+        imex_update<P>(a, c, cs, CMS, MD);
         decode(cs, T, Eold, qk, o, capped);
         capped_any |= capped;
+        // a cell outside the specialised rates' range does it again, whole and
+        // out of line (tested here and not before the rates: a branch ahead of
+        // them costs every cell 15 %, 0.47 against 0.40 ms on 1.3 M cells)
+        if (rare) {
+            imex_cell_rare<P>(&a, q, c);
+            return;
+        }
     } else if (MODE == M_ADAPT) {
         // split step: the flux residual first (Update_after_Adv + decode),
         // then the chemistry of the closed reactor at that state over dt
@@ -791,7 +895,7 @@ __device__ __forceinline__ void cell_body(const CellArgs &a, P *__restrict__ q, 
 }
 
 template <class P, int MODE, bool SPEC>
-__global__ void __launch_bounds__(128, 3) k_cell(CellArgs a, P *__restrict__ q)
+__global__ void __launch_bounds__(128, 3) k_cell(const __grid_constant__ CellArgs a, P *__restrict__ q)
 {
     cell_body<P, MODE, SPEC>(a, q);
 }

@@ -22,52 +22,6 @@
 
 namespace eu3d {
 
-// FP64 quotients and square roots without the compiler's out-of-line paths:
-// the hardware's approximation, one third-order step (the approximation's
-// error cubed, below 2^-60) and Markstein's final correction by the exact
-// remainder (P. Markstein, IBM J. Res. Dev. 34, 1990), which rounds as IEEE
-// division and square root do for results and reciprocals in the normal range.
-// Zero, infinite or NaN divisors give NaN.
-__device__ __forceinline__ double rcp_approx(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    return y;
-}
-__device__ __forceinline__ double rsqrt_approx(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    return y;
-}
-// 1/x within an ulp
-__device__ __forceinline__ double rcp_1ulp(double x)
-{
-    const double y = rcp_approx(x), e = __fma_rn(-x, y, 1.0);
-    return __fma_rn(y, __fma_rn(e, e, e), y);
-}
-// a/b from r = rcp_1ulp(b)
-__device__ __forceinline__ double div_by(double a, double b, double r)
-{
-    const double q = __dmul_rn(a, r);
-    return __fma_rn(__fma_rn(-b, q, a), r, q);
-}
-__device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, rcp_1ulp(b)); }
-__device__ __forceinline__ double rcp_rn(double x)
-{
-    const double y = rcp_1ulp(x);
-    return __fma_rn(__fma_rn(-x, y, 1.0), y, y);
-}
-// sqrt(x), x in the normal range or zero
-__device__ __forceinline__ double sqrt_rn(double x)
-{
-    const double y0 = rsqrt_approx(x);
-    const double e = __fma_rn(-__dmul_rn(x, y0), y0, 1.0);
-    const double y = __fma_rn(__dmul_rn(y0, e), __fma_rn(e, 0.375, 0.5), y0);
-    const double g = __dmul_rn(x, y);
-    return x == 0.0 ? x : __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
-}
-
 // Third-order WENO (Jiang and Shu, J. Comput. Phys. 126, 1996; new -- the
 // reference's WENO enum value has no scheme behind it): the state at the face
 // of cell ctr towards oth from the candidates ctr + (ctr - far)/2 and

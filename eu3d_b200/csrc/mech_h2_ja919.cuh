@@ -178,7 +178,11 @@ __device__ __forceinline__ void thermo_spec(const TPow &p, double h[NS], double 
     cp[8] = cp_r_spec<8>(p);
 }
 
-// Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s)
+// Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s).  For T in
+// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in
+// the normal range (common.cuh's div_rn); the caller takes the table-driven
+// form elsewhere.
+constexpr double FAST_T_LO = 150.0, FAST_T_HI = 1e4;
 __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[NS], const double Mc[NS],
                                                   const double Di[NS], const double PT[NS], double CMS[NS],
                                                   double MD[NS])
@@ -190,19 +194,20 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
 #pragma unroll
     for (int s = 0; s < NS; s++) {
         sDi[s] = fabs(Di[s]) < 0x1p-1022 ? 0x1p+64 : 1.0;
-        iDi[s] = Di[s] == 0.0 ? 0.0 : 1.0 / (Di[s] * sDi[s]);
+        iDi[s] = Di[s] == 0.0 ? 0.0 : rcp_rn(Di[s] * sDi[s]);
     }
-    const double tdep = 1.0 / (RU_CAL * (p.T * p.T));
+    const double rut = RU_CAL * p.T, irut = rcp_1ulp(rut), rgt = R_GAS * p.T, irgt = rcp_1ulp(rgt);
+    const double tdep = rcp_rn(RU_CAL * (p.T * p.T));
 #pragma unroll
     for (int s = 0; s < NS; s++) { Wi[s] = 0.0; MD[s] = 0.0; }
     {
         // reaction 1
-        const double kf = 0x1.6bcc41e900000p+46 * 1.0 * exp(-0x1.b5be07fcb923ap+15 / (RU_CAL * p.T));
+        const double kf = 0x1.6bcc41e900000p+46 * 1.0 * exp(div_by(-0x1.b5be07fcb923ap+15, rut, irut));
         const double dg = 0x1.0000000000000p+0 * G[0] + (-0x1.0000000000000p+0) * G[4] + (-0x1.0000000000000p+0) * G[5] + 0x1.0000000000000p+0 * G[7];
         const double rf = Mc[4] * Mc[5];
         const double rb = Mc[0] * Mc[7];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -218,12 +223,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 2
-        const double kf = 0x1.d8efef4880000p+47 * 1.0 * exp(-0x1.06a537e90ff97p+14 / (RU_CAL * p.T));
+        const double kf = 0x1.d8efef4880000p+47 * 1.0 * exp(div_by(-0x1.06a537e90ff97p+14, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[0] + 0x1.0000000000000p+0 * G[1] + 0x1.0000000000000p+0 * G[3] + (-0x1.0000000000000p+0) * G[4];
         const double rf = Mc[0] * Mc[4];
         const double rb = Mc[1] * Mc[3];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -239,12 +244,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 3
-        const double kf = 0x1.0c388d0000000p+34 * p.T * exp(-0x1.1647837b4a234p+13 / (RU_CAL * p.T));
+        const double kf = 0x1.0c388d0000000p+34 * p.T * exp(div_by(-0x1.1647837b4a234p+13, rut, irut));
         const double dg = 0x1.0000000000000p+0 * G[0] + (-0x1.0000000000000p+0) * G[1] + 0x1.0000000000000p+0 * G[3] + (-0x1.0000000000000p+0) * G[5];
         const double rf = Mc[1] * Mc[5];
         const double rb = Mc[0] * Mc[3];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -260,12 +265,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 4
-        const double kf = 0x1.402462f600000p+44 * 1.0 * exp(-0x1.420d8e8a71de7p+12 / (RU_CAL * p.T));
+        const double kf = 0x1.402462f600000p+44 * 1.0 * exp(div_by(-0x1.420d8e8a71de7p+12, rut, irut));
         const double dg = 0x1.0000000000000p+0 * G[0] + 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+0) * G[3] + (-0x1.0000000000000p+0) * G[5];
         const double rf = Mc[3] * Mc[5];
         const double rb = Mc[0] * Mc[2];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -281,12 +286,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 5
-        const double kf = 0x1.6eb550c600000p+42 * 1.0 * exp(-0x1.10a6b1c432ca5p+10 / (RU_CAL * p.T));
+        const double kf = 0x1.6eb550c600000p+42 * 1.0 * exp(div_by(-0x1.10a6b1c432ca5p+10, rut, irut));
         const double dg = 0x1.0000000000000p+0 * G[1] + 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+1) * G[3];
         const double rf = (Mc[3] * Mc[3]);
         const double rb = Mc[1] * Mc[2];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -304,8 +309,8 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
         const double dg = (-0x1.0000000000000p+0) * G[0] + 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+0) * G[3];
         const double rf = Mc[0] * Mc[3];
         const double rb = Mc[2];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.3bd0c106c229dp+3;
-        const double kb = kf / (kp * (R_GAS * p.T));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.3bd0c106c229dp+3;
+        const double kb = div_rn(kf, kp * (R_GAS * p.T));
         double tb = Mc[0] + Mc[1] + Mc[2] * 0x1.8000000000000p+2 + Mc[3] + Mc[4] + Mc[5] + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -323,8 +328,8 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
         const double dg = (-0x1.0000000000000p+1) * G[0] + 0x1.0000000000000p+0 * G[5];
         const double rf = (Mc[0] * Mc[0]);
         const double rb = Mc[5];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.3bd0c106c229dp+3;
-        const double kb = kf / (kp * (R_GAS * p.T));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.3bd0c106c229dp+3;
+        const double kb = div_rn(kf, kp * (R_GAS * p.T));
         double tb = Mc[0] + Mc[1] + Mc[2] * 0x1.8000000000000p+2 + Mc[3] + Mc[4] + Mc[5] * 0x1.0000000000000p+1 + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -340,8 +345,8 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
         const double dg = (-0x1.0000000000000p+0) * G[0] + (-0x1.0000000000000p+0) * G[1] + 0x1.0000000000000p+0 * G[3];
         const double rf = Mc[0] * Mc[1];
         const double rb = Mc[3];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.3bd0c106c229dp+3;
-        const double kb = kf / (kp * (R_GAS * p.T));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.3bd0c106c229dp+3;
+        const double kb = div_rn(kf, kp * (R_GAS * p.T));
         double tb = Mc[0] + Mc[1] + Mc[2] * 0x1.4000000000000p+2 + Mc[3] + Mc[4] + Mc[5] + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -355,12 +360,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 9
-        const double kf = 0x1.dd7c1681d0000p+50 * 1.0 * exp(-(-0x1.f446e2eb1c433p+9) / (RU_CAL * p.T));
+        const double kf = 0x1.dd7c1681d0000p+50 * 1.0 * exp(div_by(-(-0x1.f446e2eb1c433p+9), rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[0] + (-0x1.0000000000000p+0) * G[4] + 0x1.0000000000000p+0 * G[7];
         const double rf = Mc[0] * Mc[4];
         const double rb = Mc[7];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.3bd0c106c229dp+3;
-        const double kb = kf / (kp * (R_GAS * p.T));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.3bd0c106c229dp+3;
+        const double kb = div_rn(kf, kp * (R_GAS * p.T));
         double tb = Mc[0] + Mc[1] + Mc[2] * 0x1.0000000000000p+4 + Mc[3] + Mc[4] + Mc[5] * 0x1.0000000000000p+1 + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -374,12 +379,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 10
-        const double kf = 0x1.b48eb57e00000p+45 * 1.0 * exp(-(-0x1.c23fcd35a8588p+10) / (RU_CAL * p.T));
+        const double kf = 0x1.b48eb57e00000p+45 * 1.0 * exp(div_by(-(-0x1.c23fcd35a8588p+10), rut, irut));
         const double dg = (-0x1.0000000000000p+1) * G[1] + 0x1.0000000000000p+0 * G[4];
         const double rf = (Mc[1] * Mc[1]);
         const double rb = Mc[4];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.3bd0c106c229dp+3;
-        const double kb = kf / (kp * (R_GAS * p.T));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.3bd0c106c229dp+3;
+        const double kb = div_rn(kf, kp * (R_GAS * p.T));
         double tb = Mc[0] + Mc[1] + Mc[2] + Mc[3] + Mc[4] + Mc[5] + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -391,12 +396,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 11
-        const double kf = 0x1.fd51291300000p+46 * 1.0 * exp(-0x1.0e25c5d638866p+10 / (RU_CAL * p.T));
+        const double kf = 0x1.fd51291300000p+46 * 1.0 * exp(div_by(-0x1.0e25c5d638866p+10, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[0] + 0x1.0000000000000p+1 * G[3] + (-0x1.0000000000000p+0) * G[7];
         const double rf = Mc[0] * Mc[7];
         const double rb = (Mc[3] * Mc[3]);
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -410,12 +415,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 12
-        const double kf = 0x1.2309ce5400000p+43 * 1.0 * exp(-0x1.0e25c5d638866p+10 / (RU_CAL * p.T));
+        const double kf = 0x1.2309ce5400000p+43 * 1.0 * exp(div_by(-0x1.0e25c5d638866p+10, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[0] + 0x1.0000000000000p+0 * G[1] + 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+0) * G[7];
         const double rf = Mc[0] * Mc[7];
         const double rb = Mc[1] * Mc[2];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -431,12 +436,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 13
-        const double kf = 0x1.b48eb57e00000p+43 * 1.0 * exp(-0x1.db42b367a0f91p+9 / (RU_CAL * p.T));
+        const double kf = 0x1.b48eb57e00000p+43 * 1.0 * exp(div_by(-0x1.db42b367a0f91p+9, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[1] + 0x1.0000000000000p+0 * G[3] + 0x1.0000000000000p+0 * G[4] + (-0x1.0000000000000p+0) * G[7];
         const double rf = Mc[1] * Mc[7];
         const double rb = Mc[3] * Mc[4];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -456,8 +461,8 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
         const double dg = 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+0) * G[3] + 0x1.0000000000000p+0 * G[4] + (-0x1.0000000000000p+0) * G[7];
         const double rf = Mc[3] * Mc[7];
         const double rb = Mc[2] * Mc[4];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -477,8 +482,8 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
         const double dg = 0x1.0000000000000p+0 * G[4] + 0x1.0000000000000p+0 * G[6] + (-0x1.0000000000000p+1) * G[7];
         const double rf = (Mc[7] * Mc[7]);
         const double rb = Mc[4] * Mc[6];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -492,12 +497,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 16
-        const double kf = 0x1.45f680b000000p+40 * 1.0 * exp(-0x1.c23fcd35a8588p+11 / (RU_CAL * p.T));
+        const double kf = 0x1.45f680b000000p+40 * 1.0 * exp(div_by(-0x1.c23fcd35a8588p+11, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[0] + 0x1.0000000000000p+0 * G[5] + (-0x1.0000000000000p+0) * G[6] + 0x1.0000000000000p+0 * G[7];
         const double rf = Mc[0] * Mc[6];
         const double rb = Mc[5] * Mc[7];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -513,12 +518,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 17
-        const double kf = 0x1.977420dc00000p+43 * 1.0 * exp(-0x1.9038b6ae7d567p+12 / (RU_CAL * p.T));
+        const double kf = 0x1.977420dc00000p+43 * 1.0 * exp(div_by(-0x1.9038b6ae7d567p+12, rut, irut));
         const double dg = (-0x1.0000000000000p+0) * G[1] + 0x1.0000000000000p+0 * G[3] + (-0x1.0000000000000p+0) * G[6] + 0x1.0000000000000p+0 * G[7];
         const double rf = Mc[1] * Mc[6];
         const double rb = Mc[3] * Mc[7];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -534,12 +539,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 18
-        const double kf = 0x1.6311155200000p+42 * 1.0 * exp(-0x1.65b3212d77319p+10 / (RU_CAL * p.T));
+        const double kf = 0x1.6311155200000p+42 * 1.0 * exp(div_by(-0x1.65b3212d77319p+10, rut, irut));
         const double dg = 0x1.0000000000000p+0 * G[2] + (-0x1.0000000000000p+0) * G[3] + (-0x1.0000000000000p+0) * G[6] + 0x1.0000000000000p+0 * G[7];
         const double rf = Mc[3] * Mc[6];
         const double rb = Mc[2] * Mc[7];
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.0000000000000p+0;
-        const double kb = kf / (kp);
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.0000000000000p+0;
+        const double kb = div_rn(kf, kp);
         double tb = 0.0;
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
@@ -555,12 +560,12 @@ __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[
     }
     {
         // reaction 19
-        const double kf = 0x1.aa535d3d0c000p+56 * 1.0 * exp(-0x1.63aa6b923a29cp+15 / (RU_CAL * p.T));
+        const double kf = 0x1.aa535d3d0c000p+56 * 1.0 * exp(div_by(-0x1.63aa6b923a29cp+15, rut, irut));
         const double dg = 0x1.0000000000000p+1 * G[3] + (-0x1.0000000000000p+0) * G[6];
         const double rf = Mc[6];
         const double rb = (Mc[3] * Mc[3]);
-        const double kp = exp(-dg / (R_GAS * p.T)) * 0x1.9f06f69446738p-4;
-        const double kb = kf / (kp * (1.0 / (R_GAS * p.T)));
+        const double kp = exp(div_by(-dg, rgt, irgt)) * 0x1.9f06f69446738p-4;
+        const double kb = div_rn(kf, kp * (1.0 / (R_GAS * p.T)));
         double tb = Mc[0] + Mc[1] + Mc[2] * 0x1.e000000000000p+3 + Mc[3] + Mc[4] + Mc[5] + Mc[6] + Mc[7] + Mc[8];
         if (tb == 0.0) tb = 1.0;
         const double rr = kf * rf - kb * rb;
