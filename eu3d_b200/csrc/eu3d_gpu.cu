@@ -23,6 +23,7 @@
 #include "flux.cuh"
 #include "mlp.cuh"
 #include "surrogate.cuh"
+#include "train.cuh"
 #include "tecplot.cuh"
 #include "dlb.cuh"
 

@@ -1,7 +1,7 @@
 // Host side of the learned chemistry surrogate (C ABI in include/eu3d_gpu.h):
-// the training set on the device, FP64 labelling, the training loop over
-// the tensor-core GEMM and the elementwise kernels of mlp.cuh with Adam,
-// inference, and the coupled chemistry step of a flowfield handle.
+// the training set on the device, FP64 labelling, the training loop over the
+// kernels of train.cuh, inference, and the coupled chemistry step of a
+// flowfield handle.
 // Included once, at the end of eu3d_gpu.cu (one translation unit).
 #pragma once
 
@@ -23,13 +23,11 @@ struct eu3d_surrogate {
     float norm_h[EU3D_SUR_NORM_LEN] = {};
     SurNorm *norm_d = nullptr;
     int *err = nullptr;
-    // training buffers for batch B
+    // training: per-block gradient partials and pre-activations of a batch of B,
+    // and the batch arrays of eu3d_sur_loss_grad
     int B = 0;
-    float *Xb = nullptr, *Yb = nullptr, *acc = nullptr, *Z[3] = {}, *out4 = nullptr, *dH = nullptr, *dW[4] = {},
-          *db[4] = {}, *loss = nullptr;
+    float *part = nullptr, *zbuf = nullptr, *Xb = nullptr, *Yb = nullptr, *out4 = nullptr, *loss = nullptr;
     int loss_cap = 0;
-    __nv_bfloat16 *H0 = nullptr, *H0t = nullptr, *H[3] = {}, *Ht[3] = {}, *dZ4 = nullptr, *dZ4t = nullptr,
-                  *dZ = nullptr, *dZt = nullptr;
     std::vector<void *> train_bufs;
     // standalone inference staging
     float *in_d = nullptr, *out_d = nullptr;
@@ -40,7 +38,7 @@ namespace {
 
 const int SUR_W_IN[4] = {SUR_IN, SUR_H, SUR_H, SUR_H};
 const int SUR_W_OUT[4] = {SUR_H, SUR_H, SUR_H, SUR_OUT};
-constexpr int SUR_SPLITK = 256;  // batch rows per split-K block of the weight-gradient GEMMs
+constexpr int SUR_BATCH_ROWS = 256;  // a batch is a multiple of this
 
 void sur_free_train(eu3d_surrogate *s)
 {
@@ -77,93 +75,59 @@ int sur_alloc(eu3d_surrogate *s, T **ptr, size_t count, bool zero = true)
     return EU3D_OK;
 }
 
+// blocks of the training kernel: one per 128 rows, at most one per SM
+int sur_train_grid(const eu3d_surrogate *s, int B)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev);
+    return std::max(1, std::min(sms, B / 128));
+}
+
+// training buffers of a batch of B rows
 int sur_ensure_batch(eu3d_surrogate *s, int B)
 {
     if (s->B == B) return EU3D_OK;
     sur_free_train(s);
     int rc;
+    const int grid = sur_train_grid(s, B);
 #define SA(ptr, n) \
     if ((rc = sur_alloc(s, &(ptr), (size_t)(n)))) return rc
+    SA(s->part, (size_t)grid * TRN_PART);
+    SA(s->zbuf, (size_t)grid * TRN_Z);
     SA(s->Xb, (size_t)B * SUR_IN);
     SA(s->Yb, (size_t)B * SUR_OUT);
-    SA(s->acc, (size_t)B * SUR_H);
-    for (int l = 0; l < 3; l++) {
-        SA(s->Z[l], (size_t)B * SUR_H);
-        SA(s->H[l], (size_t)B * SUR_H);
-        SA(s->Ht[l], (size_t)B * SUR_H);
-    }
     SA(s->out4, (size_t)B * SUR_OUT);
-    SA(s->dH, (size_t)B * SUR_H);
-    SA(s->H0, (size_t)B * SUR_IN);
-    SA(s->H0t, (size_t)SUR_H * B);  // rows 16..127 stay zero (M padding of the dW1 GEMM)
-    SA(s->dZ4, (size_t)B * SUR_OUT);
-    SA(s->dZ4t, (size_t)SUR_OUT * B);
-    SA(s->dZ, (size_t)B * SUR_H);
-    SA(s->dZt, (size_t)SUR_H * B);
-    for (int l = 0; l < 4; l++) {
-        SA(s->dW[l], (size_t)SUR_H * SUR_W_OUT[l]);
-        SA(s->db[l], (size_t)SUR_W_OUT[l]);
-    }
 #undef SA
     s->B = B;
     return EU3D_OK;
 }
 
-void sur_gemm(eu3d_surrogate *s, const __nv_bfloat16 *A, const __nv_bfloat16 *Bm, float *C, int M, int N, int K,
-              bool splitk)
-{
-    if (splitk) {
-        const int ns = (K + SUR_SPLITK - 1) / SUR_SPLITK;
-        cudaMemsetAsync(C, 0, (size_t)M * N * sizeof(float), s->st);
-        k_gemm_tc<<<dim3(M / 128, ns), 128, gemm_smem_bytes(), s->st>>>(A, Bm, C, M, N, K, 0, s->err, SUR_SPLITK);
-    } else {
-        k_gemm_tc<<<M / 128, 128, gemm_smem_bytes(), s->st>>>(A, Bm, C, M, N, K, 0, s->err, 0);
-    }
-}
-
-int ew_blocks(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 16); }
-
-// forward + loss + backward on the batch already in Xb / Yb; gradient to s->g
-void sur_fwd_bwd(eu3d_surrogate *s, float *loss_slot)
-{
-    const int B = s->B;
-    cudaStream_t st = s->st;
-    const long long nh = (long long)B * SUR_H;
-    const float *bias[4] = {s->p + SUR_OFF_B1, s->p + SUR_OFF_B2, s->p + SUR_OFF_B3, s->p + SUR_OFF_B4};
-    k_sur_input<<<ew_blocks((long long)B * SUR_IN), 256, 0, st>>>(s->Xb, s->H0, s->H0t, B);
-    const __nv_bfloat16 *in = s->H0;
-    for (int l = 0; l < 3; l++) {
-        sur_gemm(s, in, s->Wt[l], s->acc, B, SUR_H, SUR_W_IN[l], false);
-        k_sur_fwd_act<<<ew_blocks(nh), 256, 0, st>>>(s->acc, bias[l], s->Z[l], s->H[l], s->Ht[l], B, SUR_H);
-        in = s->H[l];
-    }
-    sur_gemm(s, in, s->Wt[3], s->acc, B, SUR_OUT, SUR_H, false);
-    k_sur_loss<<<ew_blocks((long long)B * SUR_OUT), 256, 0, st>>>(s->acc, bias[3], s->Yb, s->out4, s->dZ4, s->dZ4t,
-                                                                  loss_slot, B);
-    // layer 4
-    sur_gemm(s, s->Ht[2], s->dZ4t, s->dW[3], SUR_H, SUR_OUT, B, true);
-    k_sur_colsum<<<SUR_OUT, 256, 0, st>>>(s->dZ4t, s->db[3], B);
-    sur_gemm(s, s->dZ4, s->W[3], s->dH, B, SUR_H, SUR_OUT, false);
-    // layers 3, 2, 1
-    for (int l = 2; l >= 0; l--) {
-        k_sur_bwd_act<<<ew_blocks(nh), 256, 0, st>>>(s->dH, s->Z[l], s->dZ, s->dZt, B, SUR_H);
-        const __nv_bfloat16 *At = l > 0 ? s->Ht[l - 1] : s->H0t;
-        sur_gemm(s, At, s->dZt, s->dW[l], SUR_H, SUR_H, B, true);
-        k_sur_colsum<<<SUR_H, 256, 0, st>>>(s->dZt, s->db[l], B);
-        if (l > 0) sur_gemm(s, s->dZ, s->W[l], s->dH, B, SUR_H, SUR_H, false);
-    }
-    k_sur_gather_grads<<<ew_blocks(SUR_NPARAM), 256, 0, st>>>(s->dW[0], s->dW[1], s->dW[2], s->dW[3], s->db[0],
-                                                             s->db[1], s->db[2], s->db[3], s->g);
-}
-
-void sur_refresh(eu3d_surrogate *s)
+SurBf16 sur_bf16(const eu3d_surrogate *s)
 {
     SurBf16 w;
     for (int l = 0; l < 4; l++) {
         w.W[l] = s->W[l];
         w.Wt[l] = s->Wt[l];
     }
-    k_sur_refresh_bf16<<<64, 256, 0, s->st>>>(s->p, w);
+    return w;
+}
+
+// forward, loss and backward of the batch in Xb / Yb, then the sum over blocks:
+// Adam, or the gradient in s->g.  next: the batch that the second kernel makes
+// for the step after (B = 0: none)
+void sur_train_step(eu3d_surrogate *s, float *out4, float *loss, const AdamCfg &adam, const BatchSrc &next, const SurNorm &nrm)
+{
+    const int grid = sur_train_grid(s, s->B);
+    k_sur_train<<<grid, TRN_THREADS, TrainSmem::BYTES + 128, s->st>>>(s->Xb, s->Yb, sur_bf16(s), s->p, s->zbuf, s->part,
+                                                                     out4, s->B, s->err);
+    const int blocks = STEP_BLOCKS + (int)(((long long)next.B * BATCH_TASKS + 255) / 256);
+    k_sur_step<<<blocks, 4 * STEP_PARAMS, 0, s->st>>>(s->part, grid, s->p, s->m, s->v, adam.update ? nullptr : s->g, loss,
+                                                     sur_bf16(s), adam, next, nrm);
+}
+
+void sur_refresh(eu3d_surrogate *s)
+{
+    k_sur_refresh_bf16<<<64, 256, 0, s->st>>>(s->p, sur_bf16(s));
 }
 
 SurWeights sur_weights(const eu3d_surrogate *s)
@@ -210,7 +174,7 @@ int sur_set_attrs()
 {
     static bool done = false;
     if (done) return EU3D_OK;
-    CK(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes()));
+    CK(cudaFuncSetAttribute(k_sur_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TrainSmem::BYTES + 128));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcArray>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcField<float>>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcField<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));
@@ -577,7 +541,7 @@ int eu3d_sur_train(eu3d_surrogate *s, int steps, int batch, float lr_max, float 
                    unsigned long long seed, float *losses)
 {
     if (!s) return fail(EU3D_ERR_ARG, "null surrogate");
-    if (steps < 0 || batch < 128 || batch % SUR_SPLITK != 0) return fail(EU3D_ERR_ARG, "batch must be a multiple of 256");
+    if (steps < 0 || batch < 128 || batch % SUR_BATCH_ROWS != 0) return fail(EU3D_ERR_ARG, "batch must be a multiple of 256");
     if (s->n < 1) return fail(EU3D_ERR_STATE, "empty training set");
     CK(cudaSetDevice(s->dev));
     int rc;
@@ -592,6 +556,9 @@ int eu3d_sur_train(eu3d_surrogate *s, int steps, int batch, float lr_max, float 
     CK(cudaMemsetAsync(s->loss, 0, (size_t)(steps + 1) * sizeof(float), s->st));
     SurNorm nrm;
     memcpy(nrm.v, s->norm_h, sizeof(nrm.v));
+    auto batch_of = [&](long long step) { return BatchSrc{s->X, s->Lb, s->n, seed, step, batch, s->Xb, s->Yb}; };
+    if (steps > 0)
+        k_sur_batch<<<(unsigned)(((long long)batch * BATCH_TASKS + 255) / 256), 256, 0, s->st>>>(batch_of(s->adam_t), nrm);
     for (int it = 0; it < steps; it++) {
         float lr = lr_max;
         if (it < warmup) {
@@ -600,12 +567,11 @@ int eu3d_sur_train(eu3d_surrogate *s, int steps, int batch, float lr_max, float 
             const double f = (double)(it - warmup) / (double)(steps - warmup);
             lr = (float)(lr_min + 0.5 * (lr_max - lr_min) * (1.0 + cos(M_PI * f)));
         }
-        k_sur_batch<<<(batch + 127) / 128, 128, 0, s->st>>>(s->X, s->Lb, s->n, nrm, seed, (long long)s->adam_t, batch,
-                                                            s->Xb, s->Yb);
-        sur_fwd_bwd(s, s->loss + it);
         s->adam_t++;
-        k_sur_adam<<<ew_blocks(SUR_NPARAM), 256, 0, s->st>>>(s->p, s->g, s->m, s->v, lr, 0.9f, 0.999f, 1e-8f, s->adam_t);
-        sur_refresh(s);
+        // the batch of the step after, drawn by its step number as this one's was
+        BatchSrc next = batch_of(s->adam_t);
+        if (it + 1 == steps) next.B = 0;
+        sur_train_step(s, nullptr, s->loss + it, AdamCfg{lr, 0.9f, 0.999f, 1e-8f, s->adam_t, 1}, next, nrm);
     }
     CK(cudaGetLastError());
     if (losses && steps > 0)
@@ -618,7 +584,7 @@ int eu3d_sur_loss_grad(eu3d_surrogate *s, const float *Xb, const float *Yb, int 
                        float *out)
 {
     if (!s || !Xb || !Yb) return fail(EU3D_ERR_ARG, "null argument");
-    if (batch < 256 || batch % SUR_SPLITK != 0) return fail(EU3D_ERR_ARG, "batch must be a multiple of 256");
+    if (batch < 256 || batch % SUR_BATCH_ROWS != 0) return fail(EU3D_ERR_ARG, "batch must be a multiple of 256");
     CK(cudaSetDevice(s->dev));
     int rc;
     if ((rc = sur_ensure_batch(s, batch))) return rc;
@@ -629,7 +595,9 @@ int eu3d_sur_loss_grad(eu3d_surrogate *s, const float *Xb, const float *Yb, int 
     CK(cudaMemcpyAsync(s->Xb, Xb, (size_t)batch * SUR_IN * sizeof(float), cudaMemcpyHostToDevice, s->st));
     CK(cudaMemcpyAsync(s->Yb, Yb, (size_t)batch * SUR_OUT * sizeof(float), cudaMemcpyHostToDevice, s->st));
     CK(cudaMemsetAsync(s->loss, 0, sizeof(float), s->st));
-    sur_fwd_bwd(s, s->loss);
+    SurNorm nrm;
+    memcpy(nrm.v, s->norm_h, sizeof(nrm.v));
+    sur_train_step(s, s->out4, s->loss, AdamCfg{}, BatchSrc{}, nrm);
     CK(cudaGetLastError());
     if (loss) CK(cudaMemcpyAsync(loss, s->loss, sizeof(float), cudaMemcpyDeviceToHost, s->st));
     if (grad) CK(cudaMemcpyAsync(grad, s->g, SUR_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, s->st));

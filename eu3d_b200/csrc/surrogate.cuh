@@ -306,35 +306,25 @@ __device__ __forceinline__ void sur_features(const SurNorm &n, const float raw[S
     f[15] = 0.f;
 }
 
-// Random minibatch (with replacement): normalised features (B x 16) and
-// standardised targets (B x 16, column 15 = sample weight).
-__global__ void k_sur_batch(const float *__restrict__ X, const float *__restrict__ Lb, long long n, SurNorm nrm,
-                            unsigned long long seed, long long step, int B, float *__restrict__ Xb,
-                            float *__restrict__ Yb)
+// Standardised target k of one training sample (raw features x, label l):
+// what its ten targets share, then each.
+struct SurTargetScale {
+    double T, sc, delta;
+};
+
+__device__ __forceinline__ SurTargetScale sur_target_scale(const SurNorm &nrm, const float *__restrict__ x)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B) return;
-    const long long idx = (long long)(smix64(seed ^ smix64((unsigned long long)step * 0x100000001ull + r)) % n);
-    float raw[SUR_NIN], f[SUR_IN];
-#pragma unroll
-    for (int i = 0; i < SUR_NIN; i++) raw[i] = X[idx * 12 + i];
-    sur_features(nrm, raw, f);
-#pragma unroll
-    for (int i = 0; i < SUR_IN; i++) Xb[(long long)r * SUR_IN + i] = f[i];
-    const double T = raw[0], dt = exp((double)raw[11]);
-    const double sc = dt * sur_activity(nrm, T);
-    const double delta = nrm.v[SN_DELTA];
-    const float *l = Lb + idx * 12;
-    float *y = Yb + (long long)r * SUR_OUT;
-#pragma unroll
-    for (int k = 0; k < SUR_NOUT; k++) {
-        const double rel = delta > 0 ? (k < NS ? exp((double)raw[2 + k]) - (double)SUR_YFLOOR + delta : T) : 1.0;
-        const double x = (double)l[k] / (sc * rel);
-        const double t = asinh(x / (double)nrm.v[SN_LIN + k]);
-        y[k] = (float)((t - nrm.v[SN_OUT_MEAN + k]) / nrm.v[SN_OUT_STD + k]);
-    }
-    for (int k = SUR_NOUT; k < 15; k++) y[k] = 0.f;
-    y[15] = l[10];
+    const double T = x[0];
+    return SurTargetScale{T, exp((double)x[11]) * sur_activity(nrm, T), nrm.v[SN_DELTA]};
+}
+
+__device__ __forceinline__ float sur_target(const SurNorm &nrm, const SurTargetScale &s, int k,
+                                            const float *__restrict__ x, float l)
+{
+    const double rel = s.delta > 0 ? (k < NS ? exp((double)x[2 + k]) - (double)SUR_YFLOOR + s.delta : s.T) : 1.0;
+    const double q = (double)l / (s.sc * rel);
+    const double t = asinh(q / (double)nrm.v[SN_LIN + k]);
+    return (float)((t - nrm.v[SN_OUT_MEAN + k]) / nrm.v[SN_OUT_STD + k]);
 }
 
 // normalised network output of one output -> raw label (dY_k or dT)
