@@ -2,9 +2,6 @@
 //
 // Reference: Flowfield::FieldBoundary_3dRSBI (src/Flowfield.cpp:559-773),
 // FieldBoundary_3dODM (:378-558), Flowfield::CFLcondition (:242-272).
-// The faces are filled in the reference's order -- x, then y over every i
-// (x ghosts included), then z over every i, j -- one launch per direction so
-// that each launch reads only cells the previous launches have finished.
 #pragma once
 
 #include "common.cuh"
@@ -47,152 +44,115 @@ __device__ __forceinline__ void ghost_store(const GhostArgs &a, P *q, long long 
     a.E[d] = E;
 }
 
+// All ghost cells in one launch.  The reference fills x, then y over every i,
+// then z over every i, j, each direction from the cells the one before has
+// finished; a cell of an edge or a corner is therefore its z image's y image's
+// x image.  Each thread follows that chain to the interior cell (or inflow
+// plane) at its end and applies what the chain does to it: copies, velocity
+// flips, and the wall-side thermodynamic recompute of the reflective faces
+// (src/Flowfield.cpp:409-436 pattern: D from P/(T Rgas), H, E, Gamma from T),
+// which depends on T, P and Y alone and so need be done once however often the
+// chain asks for it.  As three launches a small grid paid two more launches
+// and their drain per fill (4000 x 2 x 2: 12 us of a 75 us step).
 template <class P>
-__device__ __forceinline__ void ghost_copy(const GhostArgs &a, P *q, long long d, long long s)
-{
-    P v[NPRIM];
-    double T, E;
-    ghost_load(a, q, s, v, T, E);
-    ghost_store(a, q, d, v, T, E);
-}
-
-// mirror with the wall-side thermodynamic recompute of the reflective faces
-// (src/Flowfield.cpp:409-436 pattern): D from P/(T Rgas), H, E, Gamma from T
-template <class P>
-__device__ __forceinline__ void ghost_wall(const GhostArgs &a, P *q, long long d, long long s, bool flipv, bool flipw)
-{
-    const long long fs = a.L.fs;
-    const P u = q[PU * fs + s], v = q[PV * fs + s], w = q[PW * fs + s];
-    const P Pp = q[PP * fs + s];
-    P ys[NS];
-#pragma unroll
-    for (int sp = 0; sp < NS; sp++) ys[sp] = q[(PY + sp) * fs + s];
-    const double T = a.T[s];
-    q[PU * fs + d] = u;
-    q[PV * fs + d] = flipv ? -v : v;
-    q[PW * fs + d] = flipw ? -w : w;
-    q[PP * fs + d] = Pp;
-    a.T[d] = T;
-    const TPow p = tpow(T, a.quirks);
-    double Y[NS], rg = 0.0, cp = 0.0, h = 0.0, e = 0.0;
-#pragma unroll
-    for (int sp = 0; sp < NS; sp++) {
-        Y[sp] = (double)ys[sp];
-        q[(PY + sp) * fs + d] = ys[sp];
-    }
-#pragma unroll
-    for (int sp = 0; sp < NS; sp++) {
-        const double cpi = cM.ri[sp] * cp_r(sp, p);
-        const double hi = cM.ri[sp] * h_r(sp, p);
-        const double ei = hi - cM.ri[sp] * T;
-        rg += Y[sp] * cM.ri[sp];
-        cp += cpi * Y[sp];
-        h += Y[sp] * hi;
-        e += Y[sp] * ei;
-    }
-    const double Rgas = rg * 1000;
-    const double Cp = cp * 1000;
-    q[PD * fs + d] = (P)((double)Pp / (T * Rgas));
-    q[PH * fs + d] = (P)(h * 1000);
-    a.E[d] = e * 1000;
-    q[PG * fs + d] = (P)(Cp / (Cp - Rgas));
-}
-
-// x faces: i in [0, bc) and [ni+bc, ni+2bc), j, k interior
-template <class P>
-__global__ void k_ghost_x(GhostArgs a, P *q)
+__global__ void __launch_bounds__(128) k_ghost(GhostArgs a, P *q)
 {
     const Layout &L = a.L;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = 2 * L.bc;
-    const int n = g * L.nj * L.nk;
-    if (t >= n) return;
-    // a warp covers the bc ghost cells of consecutive rows j on one face:
-    // neighbouring lanes write neighbouring cells, the face is uniform across
-    // the warp, and the inflow planes (j fastest on the device) are read in order
-    const int gi = t % L.bc, j = L.bc + (t / L.bc) % L.nj;
-    const bool lower = (t / (L.bc * L.nj)) % 2 == 0;
-    const int k = L.bc + t / (g * L.nj);
-    const int i = lower ? gi : L.ni + L.bc + gi;
-    const long long d = L.at(i, j, k);
-    if (a.kind == EU3D_BC_RSBI) {
-        const int si = lower ? 2 * L.bc - 1 - i : 2 * (L.ni + L.bc) - 1 - i;
-        ghost_copy(a, q, d, L.at(si, j, k));
-    } else if (a.kind == EU3D_BC_TRANSMISSIVE) {
-        const int si = lower ? L.bc : L.ni + L.bc - 1;
-        ghost_copy(a, q, d, L.at(si, j, k));
-    } else if (a.kind == EU3D_BC_ODM) {
-        if (lower) {
-            const long long p = (long long)(k - L.bc) * L.nj + (j - L.bc), pl = (long long)L.nj * L.nk;
-            const long long fs = L.fs;
-            // the inflow values are all loaded before the first store
-            double in[9 + NS];
-#pragma unroll
-            for (int f = 0; f < 9 + NS; f++) in[f] = a.inflow[f * pl + p];
-            q[PU * fs + d] = (P)in[0];
-            q[PV * fs + d] = (P)in[1];
-            q[PW * fs + d] = (P)in[2];
-            q[PP * fs + d] = (P)in[3];
-            q[PD * fs + d] = (P)in[4];
-            a.T[d] = in[5];
-            q[PH * fs + d] = (P)in[6];
-            a.E[d] = in[7];
-            q[PG * fs + d] = (P)in[8];
-#pragma unroll
-            for (int s = 0; s < NS; s++) q[(PY + s) * fs + d] = (P)in[9 + s];
+    const int bc = L.bc, g = 2 * bc;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nz = L.NI * L.NJ * g, ny = L.NI * g * L.nk, nx = g * L.nj * L.nk;
+    int i, j, k;
+    if (t < nz) {
+        // z faces: every i, j
+        i = t % L.NI;
+        j = (t / L.NI) % L.NJ;
+        const int gk = t / (L.NI * L.NJ);
+        k = gk < bc ? gk : L.nk + gk;
+    } else if ((t -= nz) < ny) {
+        // y faces: every i, k interior
+        i = t % L.NI;
+        const int gj = (t / L.NI) % g;
+        j = gj < bc ? gj : L.nj + gj;
+        k = bc + t / (L.NI * g);
+    } else if ((t -= ny) < nx) {
+        // x faces: j, k interior; a warp covers the bc ghost cells of
+        // consecutive rows j on one face, so neighbouring lanes write
+        // neighbouring cells and read the inflow planes (j fastest) in order
+        const int gi = t % bc;
+        j = bc + (t / bc) % L.nj;
+        i = (t / (bc * L.nj)) % 2 == 0 ? gi : L.ni + bc + gi;
+        k = bc + t / (g * L.nj);
+    } else {
+        return;
+    }
+    const long long d = L.at(i, j, k), fs = L.fs;
+    bool wall = false, flipv = false, flipw = false, inflow = false;
+    if (k < bc || k >= L.nk + bc) {
+        k = k < bc ? 2 * bc - 1 - k : 2 * (L.nk + bc) - 1 - k;
+        if (a.kind == EU3D_BC_ODM) wall = flipw = true;
+    }
+    if (j < bc || j >= L.nj + bc) {
+        const bool lower = j < bc;
+        j = lower ? 2 * bc - 1 - j : 2 * (L.nj + bc) - 1 - j;
+        if (lower && a.kind != EU3D_BC_TRANSMISSIVE) wall = true;
+        if (lower && a.kind == EU3D_BC_ODM) flipv = true;
+    }
+    if (i < bc || i >= L.ni + bc) {
+        const bool lower = i < bc;
+        if (a.kind == EU3D_BC_TRANSMISSIVE) {
+            i = lower ? bc : L.ni + bc - 1;
+        } else if (a.kind == EU3D_BC_ODM && lower) {
+            inflow = true;
         } else {
-            ghost_wall(a, q, d, L.at(2 * (L.ni + L.bc) - 1 - i, j, k), false, false);
+            i = lower ? 2 * bc - 1 - i : 2 * (L.ni + bc) - 1 - i;
+            if (a.kind == EU3D_BC_ODM) wall = true;
         }
     }
-}
-
-// y faces: every i, j in the ghost rows, k interior
-template <class P>
-__global__ void k_ghost_y(GhostArgs a, P *q)
-{
-    const Layout &L = a.L;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = 2 * L.bc;
-    const int n = L.NI * g * L.nk;
-    if (t >= n) return;
-    const int i = t % L.NI, gj = (t / L.NI) % g, k = L.bc + t / (L.NI * g);
-    const bool lower = gj < L.bc;
-    const int j = lower ? gj : L.nj + L.bc + (gj - L.bc);
-    const long long d = L.at(i, j, k);
-    const int sj = lower ? 2 * L.bc - 1 - j : 2 * (L.nj + L.bc) - 1 - j;
-    if (a.kind == EU3D_BC_RSBI) {
-        if (lower)
-            ghost_wall(a, q, d, L.at(i, sj, k), false, false);
-        else
-            ghost_copy(a, q, d, L.at(i, sj, k));
-    } else if (a.kind == EU3D_BC_TRANSMISSIVE) {
-        ghost_copy(a, q, d, L.at(i, sj, k));
-    } else if (a.kind == EU3D_BC_ODM) {
-        if (lower)
-            ghost_wall(a, q, d, L.at(i, sj, k), true, false);
-        else
-            ghost_copy(a, q, d, L.at(i, sj, k));
+    P v[NPRIM];
+    double T, E;
+    if (inflow) {
+        const long long p = (long long)(k - bc) * L.nj + (j - bc), pl = (long long)L.nj * L.nk;
+        double in[9 + NS];
+#pragma unroll
+        for (int f = 0; f < 9 + NS; f++) in[f] = a.inflow[f * pl + p];
+        v[PU] = (P)in[0];
+        v[PV] = (P)in[1];
+        v[PW] = (P)in[2];
+        v[PP] = (P)in[3];
+        v[PD] = (P)in[4];
+        T = in[5];
+        v[PH] = (P)in[6];
+        E = in[7];
+        v[PG] = (P)in[8];
+#pragma unroll
+        for (int s = 0; s < NS; s++) v[PY + s] = (P)in[9 + s];
+    } else {
+        ghost_load(a, q, L.at(i, j, k), v, T, E);
     }
-}
-
-// z faces: every i, j, k in the ghost planes
-template <class P>
-__global__ void k_ghost_z(GhostArgs a, P *q)
-{
-    const Layout &L = a.L;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = 2 * L.bc;
-    const int n = L.NI * L.NJ * g;
-    if (t >= n) return;
-    const int i = t % L.NI, j = (t / L.NI) % L.NJ, gk = t / (L.NI * L.NJ);
-    const bool lower = gk < L.bc;
-    const int k = lower ? gk : L.nk + L.bc + (gk - L.bc);
-    const long long d = L.at(i, j, k);
-    const int sk = lower ? 2 * L.bc - 1 - k : 2 * (L.nk + L.bc) - 1 - k;
-    if (a.kind == EU3D_BC_ODM)
-        ghost_wall(a, q, d, L.at(i, j, sk), false, true);
-    else
-        ghost_copy(a, q, d, L.at(i, j, sk));
+    if (flipv) v[PV] = -v[PV];
+    if (flipw) v[PW] = -v[PW];
+    if (wall) {
+        const TPow p = tpow(T, a.quirks);
+        double rg = 0.0, cp = 0.0, h = 0.0, e = 0.0;
+#pragma unroll
+        for (int sp = 0; sp < NS; sp++) {
+            const double Y = (double)v[PY + sp];
+            const double cpi = cM.ri[sp] * cp_r(sp, p);
+            const double hi = cM.ri[sp] * h_r(sp, p);
+            const double ei = hi - cM.ri[sp] * T;
+            rg += Y * cM.ri[sp];
+            cp += cpi * Y;
+            h += Y * hi;
+            e += Y * ei;
+        }
+        const double Rgas = rg * 1000;
+        const double Cp = cp * 1000;
+        v[PD] = (P)((double)v[PP] / (T * Rgas));
+        v[PH] = (P)(h * 1000);
+        E = e * 1000;
+        v[PG] = (P)(Cp / (Cp - Rgas));
+    }
+    ghost_store(a, q, d, v, T, E);
 }
 
 // Wedge immersed boundary (new): solid cells take the state of the fluid
@@ -226,17 +186,22 @@ __global__ void k_wedge_band(GhostArgs a, P *q, const int4 *__restrict__ band, i
 // CFLcondition (src/Flowfield.cpp:242-272) as block maxima: because IEEE
 // division is monotone in the divisor, the smallest dx / (|U| + C) over the
 // cells is dx over the largest |U| + C, bit for bit; so each block keeps the
-// largest |U| + C, |V| + C, |W| + C of its cells and k_cfl_final divides
-// once.  A cell whose x time is NaN is skipped, as the reference's
+// largest |U| + C, |V| + C, |W| + C of its cells and the last block to
+// finish divides once.  A cell whose x time is NaN is skipped, as the reference's
 // comparisons skip it; NaN y or z times drop out of fmax as they drop out of
-// the reference's min.  One warp walks one (j, k) row of interior cells.
+// the reference's min.  One warp takes 128-cell segments of the (j, k) rows of
+// interior cells: a whole row per warp left a 4000 x 2 x 2 grid to four warps (41 us;
+// 5 with segments and the division in the same launch).
 // FP64 primitives: the reference's FP64 arithmetic (C = sqrt(gamma p / rho),
 // src/Flowfield.cpp:1281).  FP32 primitives: the same speeds in FP32 (the
 // inputs carry FP32 precision already), widened exactly for the maxima.
 __device__ __forceinline__ void cfl_speeds(double D, double Pp, double G, double U, double V, double W, double &ax,
                                            double &ay, double &az)
 {
-    const double C = sqrt(G * Pp / D);
+    const double x = G * Pp;
+    // straight-line quotient and root (the same bits) where they round as IEEE's
+    const bool normal = D >= 1e-290 && D <= 1e290 && fabs(x) <= 1e290;
+    const double C = normal ? sqrt_rn(div_rn(x, D)) : sqrt(x / D);
     ax = fabs(U) + C;
     ay = fabs(V) + C;
     az = fabs(W) + C;
@@ -251,136 +216,126 @@ __device__ __forceinline__ void cfl_speeds(float D, float Pp, float G, float U, 
     az = (double)__fadd_rn(fabsf(W), C);
 }
 
-constexpr int CFL_U = 4;  // cells a lane has in flight in k_cfl_partial
+constexpr int CFL_U = 4;  // cells a lane has in flight
+constexpr int CFL_WARPS = 8, CFL_SEG = 32 * CFL_U;
 
-template <class P>
-__global__ void k_cfl_partial(Layout L, const P *__restrict__ q, int use_z, const double *__restrict__ xn,
-                              const double *__restrict__ yn, double x0, double y0, double tn, int wedge_on,
-                              double *__restrict__ partial)
+// largest of each speed over the block, in thread 0
+__device__ __forceinline__ void cfl_block_max(double &sx, double &sy, double &sz)
 {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int rows = L.nj * L.nk;
-    const long long fs = L.fs;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int r = blockIdx.x * wpb + wid; r < rows; r += gridDim.x * wpb) {
-        const int j = L.bc + r % L.nj, k = L.bc + r / L.nj;
-        const double y = yn[j];
-        const long long base = L.at(0, j, k);
-        // CFL_U cells a lane at a time, all their loads issued before the
-        // first speed is formed (the maxima do not depend on the order)
-        for (int i0 = L.bc + lane; i0 < L.ni + L.bc; i0 += 32 * CFL_U) {
-            bool ok[CFL_U];
-            P vd[CFL_U], vp[CFL_U], vg[CFL_U], vu[CFL_U], vv[CFL_U], vw[CFL_U];
-#pragma unroll
-            for (int u = 0; u < CFL_U; u++) {
-                const int i = i0 + 32 * u;
-                ok[u] = i < L.ni + L.bc;
-                if (ok[u] && wedge_on) {
-                    const double x = xn[i];
-                    ok[u] = !(x > x0 && (y - y0) < (x - x0) * tn);
-                }
-                if (ok[u]) {
-                    const long long c = base + i;
-                    vd[u] = q[PD * fs + c];
-                    vp[u] = q[PP * fs + c];
-                    vg[u] = q[PG * fs + c];
-                    vu[u] = q[PU * fs + c];
-                    vv[u] = q[PV * fs + c];
-                    vw[u] = q[PW * fs + c];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < CFL_U; u++) {
-                if (!ok[u]) continue;
-                double ax, ay, az;
-                cfl_speeds(vd[u], vp[u], vg[u], vu[u], vv[u], vw[u], ax, ay, az);
-                if (isnan(ax)) continue;
-                sx = fmax(sx, ax);
-                sy = fmax(sy, ay);
-                if (use_z) sz = fmax(sz, az);
-            }
-        }
-    }
-    __shared__ double sm[3][32];
-    for (int o = 16; o > 0; o >>= 1) {
-        sx = fmax(sx, __shfl_down_sync(0xffffffffu, sx, o));
-        sy = fmax(sy, __shfl_down_sync(0xffffffffu, sy, o));
-        sz = fmax(sz, __shfl_down_sync(0xffffffffu, sz, o));
-    }
-    if (lane == 0) {
-        sm[0][wid] = sx;
-        sm[1][wid] = sy;
-        sm[2][wid] = sz;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        sx = lane < wpb ? sm[0][lane] : 0.0;
-        sy = lane < wpb ? sm[1][lane] : 0.0;
-        sz = lane < wpb ? sm[2][lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            sx = fmax(sx, __shfl_down_sync(0xffffffffu, sx, o));
-            sy = fmax(sy, __shfl_down_sync(0xffffffffu, sy, o));
-            sz = fmax(sz, __shfl_down_sync(0xffffffffu, sz, o));
-        }
-        if (lane == 0) {
-            partial[3 * blockIdx.x + 0] = sx;
-            partial[3 * blockIdx.x + 1] = sy;
-            partial[3 * blockIdx.x + 2] = sz;
-        }
-    }
-}
-
-// advance: time += dt as well (one rank); 0 leaves time for after the
-// all-ranks minimum of dt (k_advance_time).  dt_conv starts at 1e10 as in the
-// reference, so a domain without fluid cells gets cfl * 1e10.
-__global__ void k_cfl_final(const double *partial, int nparts, double dx, double dy, double dz, int use_z, double cfl,
-                            double final_time, double *scal, int advance)
-{
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int t = threadIdx.x; t < nparts; t += blockDim.x) {
-        sx = fmax(sx, partial[3 * t + 0]);
-        sy = fmax(sy, partial[3 * t + 1]);
-        sz = fmax(sz, partial[3 * t + 2]);
-    }
-    __shared__ double sm[3][32];
+    __shared__ double sm[3][CFL_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) {
         sx = fmax(sx, __shfl_down_sync(0xffffffffu, sx, o));
         sy = fmax(sy, __shfl_down_sync(0xffffffffu, sy, o));
         sz = fmax(sz, __shfl_down_sync(0xffffffffu, sz, o));
     }
+    __syncthreads();
     if (lane == 0) {
         sm[0][wid] = sx;
         sm[1][wid] = sy;
         sm[2][wid] = sz;
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        sx = lane < nw ? sm[0][lane] : 0.0;
-        sy = lane < nw ? sm[1][lane] : 0.0;
-        sz = lane < nw ? sm[2][lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            sx = fmax(sx, __shfl_down_sync(0xffffffffu, sx, o));
-            sy = fmax(sy, __shfl_down_sync(0xffffffffu, sy, o));
-            sz = fmax(sz, __shfl_down_sync(0xffffffffu, sz, o));
+    if (threadIdx.x == 0)
+        for (int w = 1; w < CFL_WARPS; w++) {
+            sx = fmax(sx, sm[0][w]);
+            sy = fmax(sy, sm[1][w]);
+            sz = fmax(sz, sm[2][w]);
         }
-        if (threadIdx.x == 0) {
-            // the smallest of dx/sx, dy/sy (and dz/sz); a zero speed gives an
-            // infinite time, which the reference's 1e10 start caps
-            double m = 1e10;
-            const double a = dx / sx, b = dy / sy;
-            if (a < m) m = a;
-            if (b < m) m = b;
-            if (use_z) {
-                const double z = dz / sz;
-                if (z < m) m = z;
+}
+
+// partial: one triple per block, then (at 3 max_parts) the count of finished
+// blocks, zero between launches.  advance: time += dt as well (one rank); 0
+// leaves time for after the all-ranks minimum of dt (k_advance_time).  dt_conv
+// starts at 1e10 as in the reference, so a domain without fluid cells gets
+// cfl * 1e10.
+template <class P>
+__global__ void __launch_bounds__(32 * CFL_WARPS) k_cfl(Layout L, const P *__restrict__ q, int use_z,
+                                                        const double *__restrict__ xn, const double *__restrict__ yn,
+                                                        double x0, double y0, double tn, int wedge_on,
+                                                        double *partial, int max_parts, double dx, double dy, double dz,
+                                                        double cfl, double final_time, double *scal, int advance)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long fs = L.fs;
+    const int nseg = (L.ni + CFL_SEG - 1) / CFL_SEG;
+    const int units = L.nj * L.nk * nseg;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    for (int t = blockIdx.x * CFL_WARPS + wid; t < units; t += gridDim.x * CFL_WARPS) {
+        const int r = t / nseg, i0 = L.bc + (t - r * nseg) * CFL_SEG + lane;
+        const int j = L.bc + r % L.nj, k = L.bc + r / L.nj;
+        const double y = yn[j];
+        const long long base = L.at(0, j, k);
+        // all loads of the segment are issued before the first speed is formed
+        // (the maxima do not depend on the order)
+        bool ok[CFL_U];
+        P vd[CFL_U], vp[CFL_U], vg[CFL_U], vu[CFL_U], vv[CFL_U], vw[CFL_U];
+#pragma unroll
+        for (int u = 0; u < CFL_U; u++) {
+            const int i = i0 + 32 * u;
+            ok[u] = i < L.ni + L.bc;
+            if (ok[u] && wedge_on) {
+                const double x = xn[i];
+                ok[u] = !(x > x0 && (y - y0) < (x - x0) * tn);
             }
-            double dt = cfl * m;
-            if (scal[1] + dt > final_time) dt = final_time - scal[1];
-            scal[0] = dt;
-            if (advance) scal[1] += dt;
+            if (ok[u]) {
+                const long long c = base + i;
+                vd[u] = q[PD * fs + c];
+                vp[u] = q[PP * fs + c];
+                vg[u] = q[PG * fs + c];
+                vu[u] = q[PU * fs + c];
+                vv[u] = q[PV * fs + c];
+                vw[u] = q[PW * fs + c];
+            }
         }
+#pragma unroll
+        for (int u = 0; u < CFL_U; u++) {
+            if (!ok[u]) continue;
+            double ax, ay, az;
+            cfl_speeds(vd[u], vp[u], vg[u], vu[u], vv[u], vw[u], ax, ay, az);
+            if (isnan(ax)) continue;
+            sx = fmax(sx, ax);
+            sy = fmax(sy, ay);
+            if (use_z) sz = fmax(sz, az);
+        }
+    }
+    cfl_block_max(sx, sy, sz);
+    __shared__ bool last;
+    unsigned *done = reinterpret_cast<unsigned *>(partial + 3 * (size_t)max_parts);
+    if (threadIdx.x == 0) {
+        partial[3 * blockIdx.x + 0] = sx;
+        partial[3 * blockIdx.x + 1] = sy;
+        partial[3 * blockIdx.x + 2] = sz;
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    // the last block: every other block's triple is visible
+    __threadfence();
+    sx = sy = sz = 0.0;
+    for (int t = threadIdx.x; t < (int)gridDim.x; t += blockDim.x) {
+        sx = fmax(sx, __ldcg(partial + 3 * t + 0));
+        sy = fmax(sy, __ldcg(partial + 3 * t + 1));
+        sz = fmax(sz, __ldcg(partial + 3 * t + 2));
+    }
+    cfl_block_max(sx, sy, sz);
+    if (threadIdx.x == 0) {
+        *done = 0;
+        // the smallest of dx/sx, dy/sy (and dz/sz); a zero speed gives an
+        // infinite time, which the reference's 1e10 start caps
+        double m = 1e10;
+        const double a = dx / sx, b = dy / sy;
+        if (a < m) m = a;
+        if (b < m) m = b;
+        if (use_z) {
+            const double z = dz / sz;
+            if (z < m) m = z;
+        }
+        double dt = cfl * m;
+        if (scal[1] + dt > final_time) dt = final_time - scal[1];
+        scal[0] = dt;
+        if (advance) scal[1] += dt;
     }
 }
 

@@ -497,21 +497,9 @@ void launch_ghost(eu3d_handle *h, int kind)
     const Layout &L = h->L;
     const int g = 2 * L.bc;
     if (kind != EU3D_BC_NONE) {
-        int n = g * L.nj * L.nk;
-        {
-            ProfScope ps(h, "ghost_x");
-            k_ghost_x<P><<<(n + 255) / 256, 256, 0, h->st>>>(a, q);
-        }
-        n = L.NI * g * L.nk;
-        {
-            ProfScope ps(h, "ghost_y");
-            k_ghost_y<P><<<(n + 255) / 256, 256, 0, h->st>>>(a, q);
-        }
-        n = L.NI * L.NJ * g;
-        {
-            ProfScope ps(h, "ghost_z");
-            k_ghost_z<P><<<(n + 255) / 256, 256, 0, h->st>>>(a, q);
-        }
+        const long long n = (long long)g * (L.NI * L.NJ + L.NI * L.nk + L.nj * L.nk);
+        ProfScope ps(h, "ghost");
+        k_ghost<P><<<(unsigned)((n + 127) / 128), 128, 0, h->st>>>(a, q);
     }
     if (h->wedge_on && h->wedge_nband > 0) {
         const double tn = h->wedge[2];
@@ -543,14 +531,14 @@ template <class P>
 void launch_cfl(eu3d_handle *h, const Spacing &sp, double cfl, double final_time, int advance)
 {
     const int use_z = (h->quirks & EU3D_Q_CFL_NO_Z) ? 0 : 1;
-    {
-        ProfScope ps(h, "cfl_partial");
-        k_cfl_partial<P><<<h->cfl_parts, 256, 0, h->st>>>(h->L, (const P *)h->prim, use_z, h->xn, h->yn, h->wedge[0],
-                                                       h->wedge[1], h->wedge[2], h->wedge_on, h->partial);
-    }
-    ProfScope ps(h, "cfl_final");
-    k_cfl_final<<<1, 1024, 0, h->st>>>(h->partial, h->cfl_parts, sp.dx, sp.dy, sp.dz, use_z, cfl, final_time, h->scal,
-                                       advance);
+    // one 128-cell segment a warp while the grid has fewer than cfl_parts blocks of them
+    const Layout &L = h->L;
+    const long long units = (long long)L.nj * L.nk * ((L.ni + CFL_SEG - 1) / CFL_SEG);
+    const int blocks = (int)std::min<long long>(h->cfl_parts, (units + CFL_WARPS - 1) / CFL_WARPS);
+    ProfScope ps(h, "cfl");
+    k_cfl<P><<<blocks, 32 * CFL_WARPS, 0, h->st>>>(L, (const P *)h->prim, use_z, h->xn, h->yn, h->wedge[0], h->wedge[1],
+                                                  h->wedge[2], h->wedge_on, h->partial, h->cfl_parts, sp.dx, sp.dy, sp.dz,
+                                                  cfl, final_time, h->scal, advance);
 }
 
 Spacing g_spacing(eu3d_handle *h);
@@ -1133,7 +1121,7 @@ int eu3d_create(const eu3d_desc *d, eu3d_handle **out)
     // CFL: 16 blocks of 8 warps per SM, each warp walking a few rows, keep
     // enough loads in flight to stream the six primitive fields
     h->cfl_parts = 148 * 16;
-    ALLOC(h->partial, 3 * h->cfl_parts * sizeof(double));  // per block: largest |U|+C, |V|+C, |W|+C
+    ALLOC(h->partial, (3 * h->cfl_parts + 1) * sizeof(double));  // per block: largest |U|+C, |V|+C, |W|+C; a count
     ALLOC(h->status, sizeof(Status));
 #undef ALLOC
     cudaMemsetAsync(h->cs, 0, NV * f8, h->st);
@@ -1143,6 +1131,7 @@ int eu3d_create(const eu3d_desc *d, eu3d_handle **out)
     cudaMemsetAsync(h->prim, 0, (size_t)NPRIM * L.fs * prim_bytes(h), h->st);
     cudaMemsetAsync(h->nchem, 0, (size_t)L.fs * sizeof(int), h->st);
     cudaMemsetAsync(h->scal, 0, 8 * sizeof(double), h->st);
+    cudaMemsetAsync(h->partial, 0, (3 * h->cfl_parts + 1) * sizeof(double), h->st);
     cudaMemsetAsync(h->status, 0, sizeof(Status), h->st);
     cudaMemcpyAsync(h->xn, d->xnode, L.NI * sizeof(double), cudaMemcpyHostToDevice, h->st);
     cudaMemcpyAsync(h->yn, d->ynode, L.NJ * sizeof(double), cudaMemcpyHostToDevice, h->st);
