@@ -608,6 +608,24 @@ __device__ __forceinline__ bool solid_cell(const CellArgs &a, int i, int j)
     return x > a.wedge[0] && (y - a.wedge[1]) < (x - a.wedge[0]) * a.wedge[2];
 }
 
+// The interior cell of a thread of the one-thread-per-cell kernels: each warp
+// takes a 32-cell segment of an x row, the segments numbered through over all
+// rows, so that every block is full whatever the row length (blocks cut from
+// single rows left the second block of a 160-cell row with one warp of four).
+// False past the row's end and the last row.
+__device__ __forceinline__ bool cell_of_thread(const Layout &L, int &i, int &j, int &k)
+{
+    const unsigned nseg = ((unsigned)L.ni + 31u) >> 5;
+    const unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const unsigned row = t / nseg;
+    i = L.bc + (int)((t - row * nseg) * 32u + (threadIdx.x & 31));
+    k = (int)(row / (unsigned)L.nj);
+    j = L.bc + (int)(row - (unsigned)k * (unsigned)L.nj);
+    const bool in = k < L.nk && i < L.ni + L.bc;
+    k += L.bc;
+    return in;
+}
+
 // the flux residual of cell index i as FP64 (its storage has the primitives' precision)
 template <class P>
 __device__ __forceinline__ double rhs_at(const CellArgs &a, long long i)
@@ -729,10 +747,8 @@ template <class P, int MODE, bool SPEC, bool GOUT = false>
 __device__ __forceinline__ void cell_body(const CellArgs &a, P *__restrict__ q, CellGate *gout = nullptr)
 {
     const Layout &L = a.L;
-    const int i = L.bc + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = L.bc + blockIdx.y;
-    const int k = L.bc + blockIdx.z;
-    if (i >= L.ni + L.bc) return;
+    int i, j, k;
+    if (!cell_of_thread(L, i, j, k)) return;
     if (solid_cell(a, i, j)) return;
     const long long c = L.at(i, j, k);
     const long long fs = L.fs;
@@ -894,19 +910,25 @@ __device__ __forceinline__ void cell_body(const CellArgs &a, P *__restrict__ q, 
     warp_count(&a.st->nonfinite, !(isfinite(o.D) && isfinite(o.T)));
 }
 
-template <class P, int MODE, bool SPEC>
-__global__ void __launch_bounds__(128, 3) k_cell(const __grid_constant__ CellArgs a, P *__restrict__ q)
-{
-    cell_body<P, MODE, SPEC>(a, q);
-}
+// Threads and resident blocks a kernel of each mode is compiled for.  The
+// stage updates and the plain decode are bound by memory latency behind the
+// decode's FP64 chain: 16 warps an SM at 128 registers (1.3 M cells, FP32
+// primitives: stage 1 115 -> 103 us, stage 2 117 -> 111; FP64: 126 -> 120, 136 ->
+// 135; the same bits; 64 x 10 spills and moves the last bits).  One-step IMEX
+// wants registers (12 warps at 168) and, its code being longer than the
+// instruction cache, wide blocks whose warps fetch it together: 128 x 3 322 us,
+// 192 x 2 310, 96 x 5 356, 160 x 3 356, 416 x 1 377.
+template <int MODE>
+struct CellShape {
+    static constexpr bool stage = MODE == M_DECODE || MODE == M_ADV || MODE == M_NOCHEM || MODE == M_RK_STAGE1 ||
+                                  MODE == M_RK_STAGE2 || MODE == M_RK3_STAGE2 || MODE == M_RK3_STAGE3;
+    static constexpr int THREADS = MODE == M_IMEX ? 192 : 128;
+    static constexpr int BLOCKS = MODE == M_IMEX ? 2 : stage ? 4 : 3;
+};
 
-// The same cell update compiled for NB resident blocks of 128 threads per SM
-// (fewer registers a thread): the memory-bound SSP-RK2 stage updates, whose
-// decode otherwise holds 167 registers and leaves 12 warps per SM to cover
-// the HBM latency (tuning cell_blocks; NB = 4 gives the results of NB = 3
-// bit for bit).
-template <class P, int MODE, bool SPEC, int NB>
-__global__ void __launch_bounds__(128, NB) k_cell_nb(CellArgs a, P *__restrict__ q)
+template <class P, int MODE, bool SPEC>
+__global__ void __launch_bounds__(CellShape<MODE>::THREADS, CellShape<MODE>::BLOCKS)
+    k_cell(const __grid_constant__ CellArgs a, P *__restrict__ q)
 {
     cell_body<P, MODE, SPEC>(a, q);
 }

@@ -93,7 +93,7 @@ struct eu3d_handle {
     int sur_fused = 0;     // surrogate: network and apply in one kernel (1) or two kernels (0, faster)
     unsigned wait_tries = 1u << 19;  // bound of the flux ring's copy waits (eu3d_set_wait_limit)
     int adapt_queue = 0;   // FP64 adaptive chemistry on the persistent queue (1) or one thread per cell (0)
-    int cell_blocks = 3;   // resident blocks per SM of the FP32-path SSP-RK2 stage updates (3 or 4)
+    int cell_blocks = 3;   // accepted (3 or 4) and reported; the stage updates run at CellShape's occupancy
     int gate_fused = 1;    // surrogate with its gate: the gate runs inside SSP-RK2's stage 2 (1) or on its own (0)
     bool sur_gated = false;  // the last stage 2 listed the active cells; the next surrogate step uses that list
     AdaptCfg acfg{0.02, 0.5, 1024};  // adaptive chemistry (EU3D_REACT_ADAPTIVE, surrogate fallback)
@@ -216,38 +216,43 @@ CellArgs cell_args(eu3d_handle *h)
     return a;
 }
 
+// blocks of bx threads for kernels that take their cell from cell_of_thread
+unsigned cell_blocks_of(const Layout &L, int bx)
+{
+    const long long segs = (long long)L.nj * L.nk * ((L.ni + 31) / 32);
+    return (unsigned)((segs + bx / 32 - 1) / (bx / 32));
+}
+
 dim3 cell_grid(const Layout &L, int bx) { return dim3((L.ni + bx - 1) / bx, L.nj, L.nk); }
+
+template <class P, int MODE, bool SPEC>
+void launch_cell_mode(eu3d_handle *h, const CellArgs &a, P *q)
+{
+    constexpr int threads = CellShape<MODE>::THREADS;
+    k_cell<P, MODE, SPEC><<<cell_blocks_of(h->L, threads), threads, 0, h->st>>>(a, q);
+}
 
 template <class P, bool SPEC>
 void launch_cell_t(eu3d_handle *h, int mode)
 {
     CellArgs a = cell_args(h);
     P *q = (P *)h->prim;
-    dim3 g = cell_grid(h->L, 128);
     static const char *names[] = {"cell_decode", "cell_adv",   "cell_imex",          "cell_trap0", "cell_trap1",
                                   "cell_rk1",    "cell_rk2",   "cell_nochem",        "cell_trap1_predict",
                                   "cell_adapt",  "cell_rk3_2", "cell_rk3_3"};
     ProfScope ps(h, names[mode]);
-    if constexpr (sizeof(P) == 4) {
-        // SSP-RK2 stage updates of the FP32-flux path at the tuned occupancy
-        if ((mode == M_RK_STAGE1 || mode == M_RK_STAGE2) && h->cell_blocks == 4) {
-            if (mode == M_RK_STAGE1) k_cell_nb<P, M_RK_STAGE1, SPEC, 4><<<g, 128, 0, h->st>>>(a, q);
-            else k_cell_nb<P, M_RK_STAGE2, SPEC, 4><<<g, 128, 0, h->st>>>(a, q);
-            return;
-        }
-    }
     switch (mode) {
-    case M_DECODE: k_cell<P, M_DECODE, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_ADV: k_cell<P, M_ADV, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_IMEX: k_cell<P, M_IMEX, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_TRAP0: k_cell<P, M_TRAP0, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_TRAP1: k_cell<P, M_TRAP1, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_RK_STAGE1: k_cell<P, M_RK_STAGE1, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_RK_STAGE2: k_cell<P, M_RK_STAGE2, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_NOCHEM: k_cell<P, M_NOCHEM, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_ADAPT: k_cell<P, M_ADAPT, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_RK3_STAGE2: k_cell<P, M_RK3_STAGE2, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
-    case M_RK3_STAGE3: k_cell<P, M_RK3_STAGE3, SPEC><<<g, 128, 0, h->st>>>(a, q); break;
+    case M_DECODE: launch_cell_mode<P, M_DECODE, SPEC>(h, a, q); break;
+    case M_ADV: launch_cell_mode<P, M_ADV, SPEC>(h, a, q); break;
+    case M_IMEX: launch_cell_mode<P, M_IMEX, SPEC>(h, a, q); break;
+    case M_TRAP0: launch_cell_mode<P, M_TRAP0, SPEC>(h, a, q); break;
+    case M_TRAP1: launch_cell_mode<P, M_TRAP1, SPEC>(h, a, q); break;
+    case M_RK_STAGE1: launch_cell_mode<P, M_RK_STAGE1, SPEC>(h, a, q); break;
+    case M_RK_STAGE2: launch_cell_mode<P, M_RK_STAGE2, SPEC>(h, a, q); break;
+    case M_NOCHEM: launch_cell_mode<P, M_NOCHEM, SPEC>(h, a, q); break;
+    case M_ADAPT: launch_cell_mode<P, M_ADAPT, SPEC>(h, a, q); break;
+    case M_RK3_STAGE2: launch_cell_mode<P, M_RK3_STAGE2, SPEC>(h, a, q); break;
+    case M_RK3_STAGE3: launch_cell_mode<P, M_RK3_STAGE3, SPEC>(h, a, q); break;
     }
 }
 
@@ -269,7 +274,7 @@ void trap1_predict(eu3d_handle *h)
     h->away_lo = h->away_hi = 0;
     h->dlb_segs.n = 0;  // a new prediction: no rows selected yet
     ProfScope ps(h, "trap1_predict");
-    k_cell<P, M_TRAP1_PREDICT, SPEC><<<cell_grid(h->L, 128), 128, 0, h->st>>>(a, (P *)h->prim);
+    launch_cell_mode<P, M_TRAP1_PREDICT, SPEC>(h, a, (P *)h->prim);
 }
 
 template <class P, bool SPEC>
@@ -2216,23 +2221,17 @@ int eu3d_autotune(eu3d_handle *h, const eu3d_step_desc *s, int steps, eu3d_tunin
     std::vector<eu3d_tuning> cands;
     const bool q = s->react == EU3D_REACT_TRAPEZOID && s->type == 1;
     const bool aq = s->react == EU3D_REACT_ADAPTIVE;
-    const bool rk2 = s->timeadv == EU3D_ADV_SSPRK2 && h->flux_bits == 32;
     for (int fst : {0, 1, 2})
         for (int kz : {4, 8, 16, 32, 64})
             for (int cq : {0, 1})
                 for (int qb : {2, 3, 4})
-                    for (int ad : {0, 1})
-                        for (int cb : {3, 4}) {
-                            if (h->flux_bits == 64 && fst != start.flux_stage) continue;
-                            if (!q && (cq != start.chem_queue || qb != start.queue_blocks)) continue;
-                            if (q && cq == 0 && qb != start.queue_blocks) continue;
-                            if (!aq && ad != start.adapt_queue) continue;
-                            if (!rk2 && cb != start.cell_blocks) continue;
-                            // the stage occupancy is tuned at the default flux setting
-                            if (rk2 && cb != start.cell_blocks && (fst != start.flux_stage || kz != start.flux_kz))
-                                continue;
-                            cands.push_back({kz, cq, qb, fst, start.sur_fused, ad, cb, start.gate_fused});
-                        }
+                    for (int ad : {0, 1}) {
+                        if (h->flux_bits == 64 && fst != start.flux_stage) continue;
+                        if (!q && (cq != start.chem_queue || qb != start.queue_blocks)) continue;
+                        if (q && cq == 0 && qb != start.queue_blocks) continue;
+                        if (!aq && ad != start.adapt_queue) continue;
+                        cands.push_back({kz, cq, qb, fst, start.sur_fused, ad, start.cell_blocks, start.gate_fused});
+                    }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);

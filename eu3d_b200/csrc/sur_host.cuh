@@ -279,12 +279,9 @@ void rk2_gate_t(eu3d_handle *h)
     P *q = (P *)h->prim;
     const SurQueue qu{h->sur_list, h->sur_count, h->sur_audit, L.interior_cells(), h->sur_res, h->sur_info};
     const SurGate g{h->gate_T, (float)h->gate_y, h->gate_mask, h->gate_audit, h->sur_active, h->sur_count + 2};
-    const dim3 grid = cell_grid(L, 128);
+    const unsigned grid = cell_blocks_of(L, 128);
     ProfScope ps(h, "cell_rk2");
-    if (sizeof(P) == 4 && h->cell_blocks == 4)
-        k_rk2_gate<P, SPEC, 4><<<grid, 128, 0, h->st>>>(a, q, g, qu);
-    else
-        k_rk2_gate<P, SPEC, 3><<<grid, 128, 0, h->st>>>(a, q, g, qu);
+    k_rk2_gate<P, SPEC><<<grid, 128, 0, h->st>>>(a, q, g, qu);
 }
 
 int rk2_gate_op(eu3d_handle *h)

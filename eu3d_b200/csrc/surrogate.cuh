@@ -975,14 +975,14 @@ __global__ void __launch_bounds__(GATE_THREADS) k_sur_gate(CellArgs a, const P *
 // reading T and the radicals back from memory.  Every lane reaches its
 // warp's append (cell_body returns to this kernel for cells past the row or
 // in the wedge).
-template <class P, bool SPEC, int NB>
-__global__ void __launch_bounds__(128, NB) k_rk2_gate(CellArgs a, P *__restrict__ q, SurGate g, SurQueue qu)
+template <class P, bool SPEC>
+__global__ void __launch_bounds__(128, 4) k_rk2_gate(const __grid_constant__ CellArgs a, P *__restrict__ q, SurGate g, SurQueue qu)
 {
     CellGate gc{g.mask, false, 0, 0.0, 0.f};
     cell_body<P, M_RK_STAGE2, SPEC, true>(a, q, &gc);
     const Layout &L = a.L;
-    const int i = L.bc + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = L.bc + blockIdx.y, k = L.bc + blockIdx.z;
+    int i, j, k;
+    cell_of_thread(L, i, j, k);
     const bool frozen = gc.valid && gc.T < g.T_frozen && (!g.mask || gc.y <= g.y_max_f);
     const bool active = gc.valid && !frozen;
     // one list atomic per warp, no block barrier: a barrier would hold every

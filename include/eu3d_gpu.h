@@ -312,9 +312,9 @@ int eu3d_sdlb_unpack(eu3d_handle *h, const double *dev_back);
    adapt_queue 1: the FP64 adaptive chemistry (EU3D_REACT_ADAPTIVE) lists the
    fluid cells and integrates them on the persistent queue, one cell per lane
    with refill; 0 (default): one thread per cell.  cell_blocks (3, default,
-   or 4): resident blocks of 128 threads per SM the SSP-RK2 stage updates of
-   the FP32-flux path are compiled for (more blocks, fewer registers a
-   thread; the same results).  gate_fused (1, default): in an SSP-RK2 step
+   or 4): accepted and reported; the stage updates are compiled for four
+   resident blocks of 128 threads per SM either way, the faster of the two
+   (the same results).  gate_fused (1, default): in an SSP-RK2 step
    with the learned chemistry and its frozen-chemistry gate on, the gate runs
    inside stage 2 on the state the stage has just decoded, instead of as a
    kernel of its own that reads T and the radicals back (0); the same list
@@ -343,10 +343,8 @@ int eu3d_get_tuning(eu3d_handle *h, eu3d_tuning *t);
 /* Autotuner: times `steps` steps of s for each candidate setting (flux_kz in
    {4, 8, 16, 32, 64}, the three FP32 flux kernels; for the adaptive
    trapezoid also the queue on/off and 2..4 blocks per SM; for the FP64
-   adaptive chemistry adapt_queue on/off; for SSP-RK2 with FP32 flux the
-   stage updates' cell_blocks 3, 4) on the handle's current state,
-   restoring the state after
-   each trial, and keeps the fastest.  best / best_ms may be NULL.  Needs
+   adaptive chemistry adapt_queue on/off) on the handle's current state,
+   restoring the state after each trial, and keeps the fastest.  best / best_ms may be NULL.  Needs
    temporary device memory for one copy of the state. */
 int eu3d_autotune(eu3d_handle *h, const eu3d_step_desc *s, int steps, eu3d_tuning *best, double *best_ms);
 
