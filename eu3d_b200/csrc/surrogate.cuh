@@ -1078,8 +1078,12 @@ struct SurSrcFieldApply : SurSrcField<P> {
 // one thread per slot -- run inside the loop, that work was executed by the
 // warp in nearly every pass (some lane finishes a cell in most passes), and
 // its code competed with the substep's for the instruction cache.
+// Two resident blocks (255 registers): at three the substep loop spills 770
+// bytes a thread, and the cells' uneven substep counts leave little for the third
+// block to hide (272 against 226 us on 4.2 M cells of a developed oblique
+// detonation, 318 at four).
 template <class P, bool SPEC>
-__global__ void __launch_bounds__(128, 3) k_sur_fallback(CellArgs a, P *__restrict__ q, SurQueue qu)
+__global__ void __launch_bounds__(128, 2) k_sur_fallback(CellArgs a, P *__restrict__ q, SurQueue qu)
 {
     const int lane = threadIdx.x & 31;
     const int total = (int)min((long long)*qu.count, qu.cap);
