@@ -60,6 +60,12 @@ struct StepKey {
 
 }  // namespace
 
+// node spacings the reference's CFLcondition uses: node(1) - node(0) of each
+// axis (src/Flowfield.cpp:244-246)
+struct Spacing {
+    double dx, dy, dz;
+};
+
 struct eu3d_handle {
     int dev = 0;
     cudaStream_t st = nullptr;
@@ -71,6 +77,7 @@ struct eu3d_handle {
     void *prim = nullptr;
     int *nchem = nullptr;
     double *xn = nullptr, *yn = nullptr, *zn = nullptr;
+    Spacing sp{};  // taken from the nodes at creation (read back, it cost each eu3d_cfl three blocking copies)
     double *scal = nullptr;  // [0] dt, [1] time
     double *partial = nullptr;
     int nparts = 0;     // persistent-queue blocks (fallback queue)
@@ -527,11 +534,6 @@ int ghost_op(eu3d_handle *h, int kind)
     return EU3D_OK;
 }
 
-// node spacings the reference's CFLcondition uses (src/Flowfield.cpp:244-246)
-struct Spacing {
-    double dx, dy, dz;
-};
-
 template <class P>
 void launch_cfl(eu3d_handle *h, const Spacing &sp, double cfl, double final_time, int advance)
 {
@@ -545,8 +547,6 @@ void launch_cfl(eu3d_handle *h, const Spacing &sp, double cfl, double final_time
                                                   h->wedge[2], h->wedge_on, h->partial, h->cfl_parts, sp.dx, sp.dy, sp.dz,
                                                   cfl, final_time, h->scal, advance);
 }
-
-Spacing g_spacing(eu3d_handle *h);
 
 int cfl_op(eu3d_handle *h, double cfl, double final_time, const Spacing &sp, int advance = 1)
 {
@@ -706,20 +706,6 @@ int prim_index(int field)
 }
 
 int grid_blocks(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 32); }
-
-Spacing g_spacing(eu3d_handle *h)
-{
-    // the reference reads node(1) - node(0) of each axis (src/Flowfield.cpp:244-246)
-    Spacing s;
-    double x[2], y[2], z[2];
-    cudaMemcpy(x, h->xn, 2 * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaMemcpy(y, h->yn, 2 * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaMemcpy(z, h->zn, 2 * sizeof(double), cudaMemcpyDeviceToHost);
-    s.dx = x[1] - x[0];
-    s.dy = y[1] - y[0];
-    s.dz = z[1] - z[0];
-    return s;
-}
 
 int validate_mech(const eu3d_desc *d, MechConst &m)
 {
@@ -1138,6 +1124,7 @@ int eu3d_create(const eu3d_desc *d, eu3d_handle **out)
     cudaMemsetAsync(h->scal, 0, 8 * sizeof(double), h->st);
     cudaMemsetAsync(h->partial, 0, (3 * h->cfl_parts + 1) * sizeof(double), h->st);
     cudaMemsetAsync(h->status, 0, sizeof(Status), h->st);
+    h->sp = Spacing{d->xnode[1] - d->xnode[0], d->ynode[1] - d->ynode[0], d->znode[1] - d->znode[0]};
     cudaMemcpyAsync(h->xn, d->xnode, L.NI * sizeof(double), cudaMemcpyHostToDevice, h->st);
     cudaMemcpyAsync(h->yn, d->ynode, L.NJ * sizeof(double), cudaMemcpyHostToDevice, h->st);
     cudaMemcpyAsync(h->zn, d->znode, L.NK * sizeof(double), cudaMemcpyHostToDevice, h->st);
@@ -1451,7 +1438,7 @@ int eu3d_get_dt(eu3d_handle *h, double *dt)
 int eu3d_cfl(eu3d_handle *h, double cfl, double final_time, double *dt_out)
 {
     if (!h) return fail(EU3D_ERR_ARG, "null handle");
-    int rc = cfl_op(h, cfl, final_time, g_spacing(h));
+    int rc = cfl_op(h, cfl, final_time, h->sp);
     if (rc) return rc;
     return dt_out ? eu3d_get_dt(h, dt_out) : EU3D_OK;
 }
@@ -1503,7 +1490,7 @@ int eu3d_halo_unpack(eu3d_handle *h, int side, const void *src)
 int eu3d_cfl_local(eu3d_handle *h, double cfl, double final_time)
 {
     if (!h) return fail(EU3D_ERR_ARG, "null handle");
-    return cfl_op(h, cfl, final_time, g_spacing(h), 0);
+    return cfl_op(h, cfl, final_time, h->sp, 0);
 }
 
 double *eu3d_dt_device(eu3d_handle *h) { return h ? h->scal : nullptr; }
@@ -1974,11 +1961,11 @@ int eu3d_step(eu3d_handle *h, const eu3d_step_desc *s)
 {
     int prc = prepare_step(h, s);
     if (prc) return prc;
-    if (h->profile) return enqueue_step(h, s, g_spacing(h));
+    if (h->profile) return enqueue_step(h, s, h->sp);
     StepKey key{s->react, s->type, s->timeadv, s->diff, s->bc_kind, s->cfl, s->final_time};
     auto it = h->graphs.find(key);
     if (it == h->graphs.end()) {
-        const Spacing sp = g_spacing(h);
+        const Spacing sp = h->sp;
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_step(h, s, sp);
