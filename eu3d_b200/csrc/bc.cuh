@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) k_ghost(GhostArgs a, P *q)
     } else {
         return;
     }
-    const long long d = L.at(i, j, k), fs = L.fs;
+    const long long d = L.at(i, j, k);
     bool wall = false, flipv = false, flipw = false, inflow = false;
     if (k < bc || k >= L.nk + bc) {
         k = k < bc ? 2 * bc - 1 - k : 2 * (L.nk + bc) - 1 - k;
