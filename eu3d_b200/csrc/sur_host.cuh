@@ -27,6 +27,7 @@ struct eu3d_surrogate {
     // and the batch arrays of eu3d_sur_loss_grad
     int B = 0;
     float *part = nullptr, *zbuf = nullptr, *Xb = nullptr, *Yb = nullptr, *out4 = nullptr, *loss = nullptr;
+    __nv_bfloat16 *dzt = nullptr;  // paired batches (trn_paired): dZ_l^T
     int loss_cap = 0;
     std::vector<void *> train_bufs;
     // standalone inference staging
@@ -75,9 +76,11 @@ int sur_alloc(eu3d_surrogate *s, T **ptr, size_t count, bool zero = true)
     return EU3D_OK;
 }
 
-// blocks of the training kernel: one per 128 rows, at most one per SM
+// blocks of the training kernel: one per chunk of a paired batch, else one per
+// 128 rows, at most one per SM
 int sur_train_grid(const eu3d_surrogate *s, int B)
 {
+    if (trn_paired(B)) return B / TRN_CHUNK;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev);
     return std::max(1, std::min(sms, B / 128));
@@ -97,6 +100,8 @@ int sur_ensure_batch(eu3d_surrogate *s, int B)
     SA(s->Xb, (size_t)B * SUR_IN);
     SA(s->Yb, (size_t)B * SUR_OUT);
     SA(s->out4, (size_t)B * SUR_OUT);
+    s->dzt = nullptr;
+    if (trn_paired(B)) SA(s->dzt, (size_t)4 * SUR_H * B);
 #undef SA
     s->B = B;
     return EU3D_OK;
@@ -119,7 +124,8 @@ void sur_train_step(eu3d_surrogate *s, float *out4, float *loss, const AdamCfg &
 {
     const int grid = sur_train_grid(s, s->B);
     k_sur_train<<<grid, TRN_THREADS, TrainSmem::BYTES + 128, s->st>>>(s->Xb, s->Yb, sur_bf16(s), s->p, s->zbuf, s->part,
-                                                                     out4, s->B, s->err);
+                                                                     out4, s->B, s->dzt, s->err);
+    if (s->dzt) k_sur_bias<<<3 * SUR_H + SUR_OUT, TRN_CHUNK, 0, s->st>>>(s->dzt, s->B, s->part);
     const int blocks = STEP_BLOCKS + (int)(((long long)next.B * BATCH_TASKS + 255) / 256);
     k_sur_step<<<blocks, 4 * STEP_PARAMS, 0, s->st>>>(s->part, grid, s->p, s->m, s->v, adam.update ? nullptr : s->g, loss,
                                                      sur_bf16(s), adam, next, nrm);

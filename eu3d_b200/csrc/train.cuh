@@ -9,7 +9,8 @@
 // the third, written by the same epilogues.  The weight gradients stay in TMEM
 // over all of a block's samples and leave once, as the block's partial; the
 // second kernel adds the partials in block order, so a step's result does not
-// depend on scheduling.
+// depend on scheduling.  Small batches give a block 256 samples and their bias
+// sums a kernel of their own (trn_paired).
 //
 // Why one kernel: the step's 1.8 GFLOP (batch 8192) take 1 us of tensor-core
 // time; as some 30 kernels (a GEMM, an activation, a column sum, ... per
@@ -102,6 +103,15 @@ __device__ __forceinline__ void trn_store_tile(unsigned char *act, unsigned char
     }
 }
 
+// column c, rows [32 quarter, 32 quarter + 32) of a transposed tile to global
+// memory
+__device__ __forceinline__ void trn_copy_col(__nv_bfloat16 *dst, const unsigned char *tr, int c, int quarter)
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        reinterpret_cast<uint4 *>(dst)[q] = *reinterpret_cast<const uint4 *>(tr + tc::op_off(128, c, 32 * quarter + 8 * q));
+}
+
 // this thread's quarter of a column sum over a transposed tile: column c, rows
 // [32 quarter, 32 quarter + 32)
 __device__ __forceinline__ float trn_colsum(const unsigned char *tr, int c, int quarter)
@@ -118,12 +128,15 @@ __device__ __forceinline__ float trn_colsum(const unsigned char *tr, int c, int 
 }
 
 // Xb, Yb: features and targets of the batch, B x 16 each (column 15 of Yb the
-// sample's weight)
+// sample's weight).  dzt: null, and block b takes the tiles b, b + gridDim.x,
+// ...; or (trn_paired) the place of dZ_l^T, [4][128][B], and block b takes the
+// tiles 2 b and 2 b + 1 and leaves the bias gradients to k_sur_bias.
 __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__restrict__ Xb, const float *__restrict__ Yb,
                                                              SurBf16 w, const float *__restrict__ p,
                                                              float *__restrict__ zbuf,
                                                              float *__restrict__ part, float *__restrict__ out4,
-                                                             int B, int *__restrict__ err)
+                                                             int B, __nv_bfloat16 *__restrict__ dzt,
+                                                             int *__restrict__ err)
 {
     using S = TrainSmem;
     extern __shared__ unsigned char trn_raw[];
@@ -214,8 +227,14 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
         trn_store_tile(sm + S::ACT, sm + tr, row, c0, h);
     };
     float *ys = reinterpret_cast<float *>(sm + S::YS);
-    const int ntiles = B / 128;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int tile_step = dzt ? 1 : gridDim.x, tile_end = dzt ? 2 * blockIdx.x + 2 : B / 128;
+    // bias gradient of layer l (0-based) from the tile of dZ^T in T3
+    auto bias_grad = [&](int l, int tile) -> float {
+        if (!dzt) return trn_colsum(sm + S::T3, tid & 127, quarter);
+        trn_copy_col(dzt + (size_t)(l * SUR_H + (tid & 127)) * B + tile * 128 + 32 * quarter, sm + S::T3, tid & 127, quarter);
+        return 0.f;
+    };
+    for (int tile = dzt ? 2 * blockIdx.x : blockIdx.x; tile < tile_end; tile += tile_step) {
         const long long r = (long long)tile * 128 + row;
         float wt = 0.f;
         if (quarter == 0) {
@@ -267,7 +286,7 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
                 *reinterpret_cast<__nv_bfloat16 *>(sm + S::DZ4T + tc::op_off(16, c, row)) = b;
             }
         }
-        const bool more = tile + (int)gridDim.x < ntiles;
+        const bool more = tile + tile_step < tile_end;
         // l = 2, 1, 0: dH of layer l's output with the weight gradient above it,
         // then dZ_l.  dW_4 = H_3^T dZ_4, dW_{l+1}^T = dZ_{l+1}^T H_l
 #pragma unroll 1
@@ -286,18 +305,22 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
             if (l == 2) {
                 // column tid & 15, rows 4 (tid >> 4) .. + 3
                 const uint2 x = *reinterpret_cast<const uint2 *>(sm + S::DZ4T + tc::op_off(16, tid & 15, 4 * (tid >> 4)));
-                db4 += (__uint_as_float(x.x << 16) + __uint_as_float(x.x & 0xffff0000u)) +
-                       (__uint_as_float(x.y << 16) + __uint_as_float(x.y & 0xffff0000u));
+                if (dzt)
+                    *reinterpret_cast<uint2 *>(dzt + (size_t)(3 * SUR_H + (tid & 15)) * B + tile * 128 + 4 * (tid >> 4)) = x;
+                else
+                    db4 += (__uint_as_float(x.x << 16) + __uint_as_float(x.x & 0xffff0000u)) +
+                           (__uint_as_float(x.y << 16) + __uint_as_float(x.y & 0xffff0000u));
             } else {
-                dbs[1] += l == 0 ? trn_colsum(sm + S::T3, tid & 127, quarter) : 0.f;
-                dbs[2] += l == 1 ? trn_colsum(sm + S::T3, tid & 127, quarter) : 0.f;
+                const float db = bias_grad(l + 1, tile);
+                dbs[1] += l == 0 ? db : 0.f;
+                dbs[2] += l == 1 ? db : 0.f;
                 if (more) trn_load_op<128, 128>(sb + wb, l == 1 ? w.Wt[1] : w.Wt[2], tid);
                 __syncthreads();  // the column sums have read dZ^T
             }
             epilogue(l, true, S::T3);
         }
         if (!good || !run([&] { trn_mma(tmem + D1, sb + S::T3, sb + S::H0T, 16, 8, !first); })) break;
-        dbs[0] += trn_colsum(sm + S::T3, tid & 127, quarter);
+        dbs[0] += bias_grad(0, tile);
         __syncthreads();
         first = false;
     }
@@ -350,6 +373,41 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
     if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
+// Batches under 16 chunks of 256 rows keep one order of sums: a chunk's weight
+// gradients are one tensor-core accumulation over its rows, the chunks add in
+// order, and a bias gradient is the sum over the chunks of each row, then a tree
+// over the 256 rows.  Adam divides by the root of the second moment and rounds
+// the weights to BF16 at each step, so that another order of the same sums moves
+// losses and parameters by 1e-4 relative within 70 steps.  One or two chunks,
+// whose sum has no other order, have always repeated bit for bit, and runs are
+// compared with earlier ones.  More chunks once met in atomics: two such runs
+// differ by 1e-7 to 5e-6 (parameters, 20 steps), this order differs from them by
+// 4e-8 to 6e-6 at 1024 to 3072 rows where 128-row partials differ by 5e-6 to
+// 2e-5, and at 4096 rows both differ by 4e-6.  From there on a block takes 128
+// rows, which keeps twice the SMs busy: 43 us a step against 82 at 4096 and 8192
+// rows (below 4096 rows 39 to 41 against the 78 to 81 us of this order).
+constexpr int TRN_CHUNK = 256, TRN_CHUNKS = 16;
+__host__ __device__ constexpr bool trn_paired(int B) { return B < TRN_CHUNKS * TRN_CHUNK; }
+
+// bias gradients of a paired batch, into the first block's partial (the others
+// hold zeros): one block per column of dzt
+__global__ void __launch_bounds__(TRN_CHUNK) k_sur_bias(const __nv_bfloat16 *__restrict__ dzt, int B, float *__restrict__ part)
+{
+    const int c = blockIdx.x, l = c / SUR_H;
+    float s = 0.f;
+    for (int r = threadIdx.x; r < B; r += TRN_CHUNK) s += __bfloat162float(dzt[(size_t)c * B + r]);
+    __shared__ float sm[TRN_CHUNK / 32];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = threadIdx.x < TRN_CHUNK / 32 ? sm[threadIdx.x] : 0.f;
+        for (int o = TRN_CHUNK / 64; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0)
+            part[(l == 0 ? SUR_OFF_B1 : l == 1 ? SUR_OFF_B2 : l == 2 ? SUR_OFF_B3 : SUR_OFF_B4) + c - l * SUR_H] = s;
+    }
+}
+
 // The minibatch of one step: row r of B is a random sample of the training set
 // (n x 12 features X, labels Lb), with replacement.
 struct BatchSrc {
@@ -397,7 +455,8 @@ struct AdamCfg {
 };
 
 // 64 parameters a block, four threads each: a quarter of the partials, their
-// loads issued together, the quarters added in order.
+// loads issued together, the quarters added in order.  (The few partials of a
+// paired batch are the first thread's, in order.)
 constexpr int STEP_PARAMS = 64, STEP_BLOCKS = SUR_NPARAM / STEP_PARAMS + 1;
 
 __global__ void __launch_bounds__(4 * STEP_PARAMS) k_sur_step(const float *__restrict__ part, int nparts,
@@ -416,7 +475,7 @@ __global__ void __launch_bounds__(4 * STEP_PARAMS) k_sur_step(const float *__res
     const int i = blockIdx.x * STEP_PARAMS + t;
     float s = 0.f;
     if (i <= SUR_NPARAM) {
-        const int n4 = (nparts + 3) / 4, e = min(nparts, (q + 1) * n4);
+        const int n4 = nparts < TRN_CHUNKS ? nparts : (nparts + 3) / 4, e = min(nparts, (q + 1) * n4);
         int b = q * n4;
         for (; b + 16 <= e; b += 16) {
             float x[16];
