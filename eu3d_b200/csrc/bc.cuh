@@ -17,9 +17,9 @@ struct GhostArgs {
 };
 
 // Every fill loads all the values it copies before its first store.  The
-// destination of a fill is never a source of the same launch (ghost cells
-// take interior cells; the wedge band's solid cells take fluid ones), so the
-// order changes nothing but the timing: the compiler, which cannot prove
+// destination of a fill is never a source of another thread of the same launch
+// (ghost cells take interior cells; the wedge band's solid cells take fluid
+// ones), so the order changes nothing but the timing: the compiler, which cannot prove
 // that the stores miss the later loads, would otherwise issue each load only
 // after the store before it, one memory round trip per field.
 template <class P>
@@ -44,15 +44,61 @@ __device__ __forceinline__ void ghost_store(const GhostArgs &a, P *q, long long 
     a.E[d] = E;
 }
 
-// All ghost cells in one launch.  The reference fills x, then y over every i,
+// the ODM inflow state of row j, k (interior indices from 0)
+template <class P>
+__device__ __forceinline__ void ghost_inflow(const GhostArgs &a, int j, int k, P v[NPRIM], double &T, double &E)
+{
+    const long long p = (long long)k * a.L.nj + j, pl = (long long)a.L.nj * a.L.nk;
+    double in[9 + NS];
+#pragma unroll
+    for (int f = 0; f < 9 + NS; f++) in[f] = a.inflow[f * pl + p];
+    v[PU] = (P)in[0];
+    v[PV] = (P)in[1];
+    v[PW] = (P)in[2];
+    v[PP] = (P)in[3];
+    v[PD] = (P)in[4];
+    T = in[5];
+    v[PH] = (P)in[6];
+    E = in[7];
+    v[PG] = (P)in[8];
+#pragma unroll
+    for (int s = 0; s < NS; s++) v[PY + s] = (P)in[9 + s];
+}
+
+// wall-side thermodynamic recompute of the reflective faces
+// (src/Flowfield.cpp:409-436 pattern): D from P/(T Rgas), H, E, Gamma from T
+template <class P>
+__device__ __forceinline__ void ghost_wall(const GhostArgs &a, P v[NPRIM], double T, double &E)
+{
+    const TPow p = tpow(T, a.quirks);
+    double rg = 0.0, cp = 0.0, h = 0.0, e = 0.0;
+#pragma unroll
+    for (int sp = 0; sp < NS; sp++) {
+        const double Y = (double)v[PY + sp];
+        const double cpi = cM.ri[sp] * cp_r(sp, p);
+        const double hi = cM.ri[sp] * h_r(sp, p);
+        const double ei = hi - cM.ri[sp] * T;
+        rg += Y * cM.ri[sp];
+        cp += cpi * Y;
+        h += Y * hi;
+        e += Y * ei;
+    }
+    const double Rgas = rg * 1000;
+    const double Cp = cp * 1000;
+    v[PD] = (P)((double)v[PP] / (T * Rgas));
+    v[PH] = (P)(h * 1000);
+    E = e * 1000;
+    v[PG] = (P)(Cp / (Cp - Rgas));
+}
+
+// All ghost cells in one launch, for extents of at least bc (so that a mirror
+// image is an interior cell; launch_ghost).  The reference fills x, then y over every i,
 // then z over every i, j, each direction from the cells the one before has
 // finished; a cell of an edge or a corner is therefore its z image's y image's
 // x image.  Each thread follows that chain to the interior cell (or inflow
 // plane) at its end and applies what the chain does to it: copies, velocity
-// flips, and the wall-side thermodynamic recompute of the reflective faces
-// (src/Flowfield.cpp:409-436 pattern: D from P/(T Rgas), H, E, Gamma from T),
-// which depends on T, P and Y alone and so need be done once however often the
-// chain asks for it.  As three launches a small grid paid two more launches
+// flips, and the wall-side recompute, which depends on T, P and Y alone and so
+// need be done once however often the chain asks for it.  As three launches a small grid paid two more launches
 // and their drain per fill (4000 x 2 x 2: 12 us of a 75 us step).
 template <class P>
 __global__ void __launch_bounds__(128) k_ghost(GhostArgs a, P *q)
@@ -110,49 +156,49 @@ __global__ void __launch_bounds__(128) k_ghost(GhostArgs a, P *q)
     }
     P v[NPRIM];
     double T, E;
-    if (inflow) {
-        const long long p = (long long)(k - bc) * L.nj + (j - bc), pl = (long long)L.nj * L.nk;
-        double in[9 + NS];
-#pragma unroll
-        for (int f = 0; f < 9 + NS; f++) in[f] = a.inflow[f * pl + p];
-        v[PU] = (P)in[0];
-        v[PV] = (P)in[1];
-        v[PW] = (P)in[2];
-        v[PP] = (P)in[3];
-        v[PD] = (P)in[4];
-        T = in[5];
-        v[PH] = (P)in[6];
-        E = in[7];
-        v[PG] = (P)in[8];
-#pragma unroll
-        for (int s = 0; s < NS; s++) v[PY + s] = (P)in[9 + s];
-    } else {
+    if (inflow)
+        ghost_inflow(a, j - bc, k - bc, v, T, E);
+    else
         ghost_load(a, q, L.at(i, j, k), v, T, E);
-    }
     if (flipv) v[PV] = -v[PV];
     if (flipw) v[PW] = -v[PW];
-    if (wall) {
-        const TPow p = tpow(T, a.quirks);
-        double rg = 0.0, cp = 0.0, h = 0.0, e = 0.0;
-#pragma unroll
-        for (int sp = 0; sp < NS; sp++) {
-            const double Y = (double)v[PY + sp];
-            const double cpi = cM.ri[sp] * cp_r(sp, p);
-            const double hi = cM.ri[sp] * h_r(sp, p);
-            const double ei = hi - cM.ri[sp] * T;
-            rg += Y * cM.ri[sp];
-            cp += cpi * Y;
-            h += Y * hi;
-            e += Y * ei;
-        }
-        const double Rgas = rg * 1000;
-        const double Cp = cp * 1000;
-        v[PD] = (P)((double)v[PP] / (T * Rgas));
-        v[PH] = (P)(h * 1000);
-        E = e * 1000;
-        v[PG] = (P)(Cp / (Cp - Rgas));
-    }
+    if (wall) ghost_wall(a, v, T, E);
     ghost_store(a, q, d, v, T, E);
+}
+
+// The ghost cells of one axis (0: x, 1: y, 2: z), one thread per grid line, in the
+// reference's order: the lower end from the outside in, then the upper from the
+// inside out.  With an extent below bc the mirror image of an outer ghost cell
+// is a ghost cell of the other end -- the lower end takes what the last fill left
+// there, the upper what this one has just stored -- so a line is one thread's.
+template <class P, int AXIS>
+__global__ void __launch_bounds__(128) k_ghost_line(GhostArgs a, P *q)
+{
+    const Layout &L = a.L;
+    const int bc = L.bc, t = blockIdx.x * blockDim.x + threadIdx.x;
+    // lines: x over interior j, k; y over all i, interior k; z over all i, j
+    const int n1 = AXIS == 0 ? L.nj : L.NI, n2 = AXIS == 2 ? L.NJ : L.nk;
+    if (t >= n1 * n2) return;
+    const int c1 = t % n1 + (AXIS == 0 ? bc : 0), c2 = t / n1 + (AXIS == 2 ? 0 : bc);
+    const int n = AXIS == 0 ? L.ni : AXIS == 1 ? L.nj : L.nk;
+    const bool odm = a.kind == EU3D_BC_ODM, transm = a.kind == EU3D_BC_TRANSMISSIVE;
+    auto cell = [&](int p) { return AXIS == 0 ? L.at(p, c1, c2) : AXIS == 1 ? L.at(c1, p, c2) : L.at(c1, c2, p); };
+    for (int g = 0; g < 2 * bc; g++) {
+        const bool lower = g < bc;
+        const int p = lower ? g : n + g;
+        P v[NPRIM];
+        double T, E;
+        if (AXIS == 0 && odm && lower) {
+            ghost_inflow(a, c1 - bc, c2 - bc, v, T, E);
+        } else {
+            const int mirror = lower ? 2 * bc - 1 - p : 2 * (n + bc) - 1 - p;
+            ghost_load(a, q, cell(AXIS == 0 && transm ? (lower ? bc : n + bc - 1) : mirror), v, T, E);
+            if (AXIS == 1 && odm && lower) v[PV] = -v[PV];
+            if (AXIS == 2 && odm) v[PW] = -v[PW];
+            if (AXIS == 0 ? odm : AXIS == 1 ? lower && !transm : odm) ghost_wall(a, v, T, E);
+        }
+        ghost_store(a, q, cell(p), v, T, E);
+    }
 }
 
 // Wedge immersed boundary (new): solid cells take the state of the fluid

@@ -508,7 +508,14 @@ void launch_ghost(eu3d_handle *h, int kind)
     P *q = (P *)h->prim;
     const Layout &L = h->L;
     const int g = 2 * L.bc;
-    if (kind != EU3D_BC_NONE) {
+    if (kind != EU3D_BC_NONE && std::min({L.ni, L.nj, L.nk}) < L.bc) {
+        // an extent of one cell: mirror images are ghost cells, filled in order
+        auto blocks = [](long long lines) { return (unsigned)((lines + 127) / 128); };
+        ProfScope ps(h, "ghost");
+        k_ghost_line<P, 0><<<blocks((long long)L.nj * L.nk), 128, 0, h->st>>>(a, q);
+        k_ghost_line<P, 1><<<blocks((long long)L.NI * L.nk), 128, 0, h->st>>>(a, q);
+        k_ghost_line<P, 2><<<blocks((long long)L.NI * L.NJ), 128, 0, h->st>>>(a, q);
+    } else if (kind != EU3D_BC_NONE) {
         const long long n = (long long)g * (L.NI * L.NJ + L.NI * L.nk + L.nj * L.nk);
         ProfScope ps(h, "ghost");
         k_ghost<P><<<(unsigned)((n + 127) / 128), 128, 0, h->st>>>(a, q);
