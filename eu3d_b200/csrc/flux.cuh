@@ -270,13 +270,14 @@ __device__ __forceinline__ double muscl2_weight(double A0, double A1, double sep
     const double kk = 1.0 / 3.0;
     const double c1 = 0.25 * (1.0 - kk), c2 = 0.25 * (1.0 + kk);
     const double Lr = div_rn(A1, A0 + seps);
-    // comparisons on the high word (the FP64 pipe is the busy one): negative
-    // numbers count as below 1, a NaN's word is positive and above it
+    // comparisons on the high word, off the FP64 pipe.  A NaN may have either
+    // sign: it passes as above 1 or below, which both make w a NaN, and only
+    // finite negatives give 0 (a quotient past the range is a NaN, never infinite)
     const int hi = __double2hiint(Lr);
     const bool lt = hi < 0x3ff00000;
     const double L1 = lt ? Lr : 1.0, L2 = lt ? 1.0 : rcp_rn(Lr);
     const double w = __fma_rn(c1, L1, __dmul_rn(__dmul_rn(c2, L2), Lr));
-    return hi < 0 ? 0.0 : w;
+    return (unsigned)hi - 0x80000000u < 0x7ff00000u ? 0.0 : w;
 }
 
 // The state of cell ctr at the face towards oth: seps = 1e-12 for a left state
