@@ -318,7 +318,7 @@ __device__ __forceinline__ void warp_sum(unsigned long long *ctr, unsigned long 
 //
 // Two forms.  The compiled-in mechanism between FAST_T_LO and FAST_T_HI takes
 // the specialised rates with common.cuh's straight-line quotients: the same
-// bits as the compiler's divisions, of which a cell has some 120, in two
+// bits (as far as stated there) as the compiler's divisions, of which a cell has some 120, in two
 // thirds of the instructions and without their branches, which kept the
 // scheduler from overlapping the 33 exponentials.  1.3 M cells: IMEX 0.85 ->
 // 0.40 ms (cold flow) and 0.69 -> 0.41 (hot), the adaptive chemistry on hot

@@ -68,11 +68,25 @@ struct Status {
 };
 
 // FP64 quotients and square roots without the compiler's out-of-line paths:
-// the hardware's approximation, one third-order step (the approximation's
-// error cubed, below 2^-60) and Markstein's final correction by the exact
-// remainder (P. Markstein, IBM J. Res. Dev. 34, 1990), which rounds as IEEE
-// division and square root do for results and reciprocals in the normal range.
-// Zero, infinite or NaN divisors give NaN.
+// the hardware's approximation, with e its residual three terms of the series of
+// (1 - e)^-1 or (1 - e)^-1/2 (what is left is of order e^3), and Markstein's
+// final correction by the exact remainder (P. Markstein, IBM J. Res. Dev. 34,
+// 1990).  They round as IEEE division and square root do for
+//     div_by, div_rn   2^-968 <= |a|, 2^-1000 <= |b| <= 2^1000, a normal quotient; or a = 0
+//     rcp_rn           2^-1000 <= x <= 2^1000
+//     sqrt_rn          2^-960 <= x, or 0
+// but for one kind of quotient.  The correction's error is the remainder's share
+// of the reciprocal's error, half an ulp and 2^-7 of an ulp more where 1/b is next
+// to a midpoint (rcp_1ulp may then be the other neighbour); with b in [1, 2) it
+// stays below the least distance of a quotient of doubles from a midpoint, 2^-106
+// / b, while b (1 + 2^-7) < 2.  For b above 1.984 a quotient at that distance may
+// come out as its other neighbour.  (Two more operations for an exactly rounded
+// reciprocal would settle these, one pair of operands in 2^60 or fewer: FP64 flux of
+// 160^3 0.84 ms against 0.78, one-step IMEX of 1.3 M cells 331 us against 309.)
+// A test holds all this to IEEE's bits: random operands, significands next to all
+// ones, quotients next to a midpoint, the ends of the ranges.  Below the
+// numerators' bound the remainder is inexact and the last bit may differ; zero,
+// infinite or NaN divisors and quotients past the range give NaN.
 __device__ __forceinline__ double rcp_approx(double x)
 {
     double y;
@@ -98,12 +112,14 @@ __device__ __forceinline__ double div_by(double a, double b, double r)
     return __fma_rn(__fma_rn(-b, q, a), r, q);
 }
 __device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, rcp_1ulp(b)); }
+// 1/x, x > 0.  The correction starts from an estimate rounded up: from below, that
+// of an all-ones divisor ends in a tie that rounds the wrong way.
 __device__ __forceinline__ double rcp_rn(double x)
 {
-    const double y = rcp_1ulp(x);
+    const double y0 = rcp_approx(x), e = __fma_rn(-x, y0, 1.0);
+    const double y = __fma_ru(y0, __fma_rn(e, e, e), y0);
     return __fma_rn(__fma_rn(-x, y, 1.0), y, y);
 }
-// sqrt(x), x in the normal range or zero
 __device__ __forceinline__ double sqrt_rn(double x)
 {
     const double y0 = rsqrt_approx(x);

@@ -257,8 +257,9 @@ __device__ __forceinline__ void face_flux_up(const float *__restrict__ qc, int f
 // of them and two square roots; compiled as they stand they made a cell 16 000
 // instructions, most in the divisions' out-of-line paths and the branches
 // around them.  The faces below give the same bits from straight-line code:
-// div_rn and sqrt_rn round as the IEEE operations do, and the limiter's cases
-// are selected,
+// div_rn, rcp_rn and sqrt_rn round as the IEEE operations do, as far as common.cuh
+// states (a difference below 2^-968 has a slope too small to count), and the
+// limiter's cases are selected,
 //     0 < Lr < 1: minmod(Lr) = Lr, minmod(1 / Lr) = 1;
 //     Lr >= 1:    minmod(Lr) = 1,  minmod(1 / Lr) = 1 / Lr;
 //     Lr <= 0:    both 0 (a NaN Lr gives a NaN state, as 0 * NaN does there).
