@@ -430,17 +430,15 @@ struct AdaptCfg {
     int nmax;
 };
 
-// One substep of chem_adaptive: cs, T advance by h, the time left trem
-// shrinks by h, the count k grows by one.  forced is set when the substep
-// cap made h longer than the controller's choice (h = dt / nmax at least,
-// the last allowed substep takes the time left).
-template <bool SPEC>
-__device__ __forceinline__ void adapt_substep(double cs[NV], double &T, double Eold, unsigned qk, double &trem, int &k,
-                                              double hmin, const AdaptCfg &cfg, Decoded &o, int &capped_any,
-                                              int &forced)
+// The substep and the species' advance over it from their rates.  forced is set
+// when the substep cap made h longer than the controller's choice (h = dt / nmax
+// at least, the last allowed substep takes the time left).  FAST: straight-line
+// quotients, for rates of the specialised form.
+template <bool FAST>
+__device__ __forceinline__ double adapt_advance(double cs[NV], const double CMS[NS], const double MD[NS], double trem,
+                                                int k, double hmin, const AdaptCfg &cfg, int &forced)
 {
-    double CMS[NS], MD[NS];
-    imex_source<SPEC>(cs, T, qk, CMS, MD, false);
+    auto quot = [](double a, double b) { return FAST ? div_rn(a, b) : a / b; };
     double D = 0.0;
 #pragma unroll
     for (int s = 0; s < NS; s++) D += cs[s];
@@ -449,15 +447,56 @@ __device__ __forceinline__ void adapt_substep(double cs[NV], double &T, double E
     for (int s = 0; s < NS; s++) {
         const double w = fabs(CMS[s]);
         // (a quotient past the largest number comes out as NaN, which fmin drops)
-        if (w > 0.0) h = fmin(h, div_rn(cfg.rel * (cs[s] + 1e-9 * D), w));
-        if (MD[s] > 0.0) h = fmin(h, div_rn(cfg.amp, MD[s]));
+        if (w > 0.0) h = fmin(h, quot(cfg.rel * (cs[s] + 1e-9 * D), w));
+        if (MD[s] > 0.0) h = fmin(h, quot(cfg.amp, MD[s]));
     }
     const double hc = h;
     h = fmin(fmax(h, hmin), trem);
     if (k == cfg.nmax - 1) h = trem;
     if (h > hc) forced = 1;
 #pragma unroll
-    for (int s = 0; s < NS; s++) cs[s] = fmax(cs[s] + div_rn(h * CMS[s], 1.0 - h * MD[s]), 0.0);
+    for (int s = 0; s < NS; s++) cs[s] = fmax(cs[s] + quot(h * CMS[s], 1.0 - h * MD[s]), 0.0);
+    return h;
+}
+
+// the same with IEEE quotients, out of line for the rare cells outside the fast
+// range
+static __device__ __noinline__ double adapt_advance_rare(double *cs, const double *CMS, const double *MD, double trem,
+                                                         int k, double hmin, const AdaptCfg *cfg, int *forced)
+{
+    return adapt_advance<false>(cs, CMS, MD, trem, k, hmin, *cfg, *forced);
+}
+
+// One substep of chem_adaptive: cs, T advance by h, the time left trem
+// shrinks by h, the count k grows by one.
+template <bool SPEC>
+__device__ __forceinline__ void adapt_substep(double cs[NV], double &T, double Eold, unsigned qk, double &trem, int &k,
+                                              double hmin, const AdaptCfg &cfg, Decoded &o, int &capped_any,
+                                              int &forced)
+{
+    double CMS[NS], MD[NS], D = 0.0, h;
+#pragma unroll
+    for (int s = 0; s < NS; s++) D += cs[s];
+    const bool rare = SPEC && !imex_fast_ok(T, D);
+    imex_source<SPEC>(cs, T, qk, CMS, MD, false);
+    if (!rare) {
+        h = adapt_advance<SPEC>(cs, CMS, MD, trem, k, hmin, cfg, forced);
+    } else {
+        const AdaptCfg cf = cfg;
+        double c[NV], cm[NS], md[NS];
+        int fr = forced;
+#pragma unroll
+        for (int v = 0; v < NV; v++) c[v] = cs[v];
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            cm[s] = CMS[s];
+            md[s] = MD[s];
+        }
+        h = adapt_advance_rare(c, cm, md, trem, k, hmin, &cf, &fr);
+        forced = fr;
+#pragma unroll
+        for (int s = 0; s < NS; s++) cs[s] = c[s];
+    }
     int cp = 0;
     decode(cs, T, Eold, qk, o, cp);
     capped_any |= cp;
@@ -677,8 +716,10 @@ __device__ __forceinline__ int adapt_split_step(const CellArgs &a, long long c, 
     return n;
 }
 
-// Flowfield::Update_IMEX, src/Flowfield.cpp:1219-1228
-template <class P>
+// Flowfield::Update_IMEX, src/Flowfield.cpp:1219-1228.  FAST: straight-line
+// quotients, for rates of the specialised form; another mechanism's rates may
+// take a denominator past the range in which those round as IEEE's.
+template <class P, bool FAST>
 __device__ __forceinline__ void imex_update(const CellArgs &a, long long c, double cs[NV], const double CMS[NS],
                                             const double MD[NS])
 {
@@ -688,7 +729,7 @@ __device__ __forceinline__ void imex_update(const CellArgs &a, long long c, doub
         double r = rhs_at<P>(a, v * a.L.fs + c);
         if (v < NS) {
             r = r + CMS[v] * dt;
-            cs[v] = cs[v] + div_rn(r, 1.0 - dt * MD[v]);
+            cs[v] = cs[v] + (FAST ? div_rn(r, 1.0 - dt * MD[v]) : r / (1.0 - dt * MD[v]));
         } else {
             cs[v] = cs[v] + r;
         }
@@ -702,15 +743,11 @@ __device__ __noinline__ void imex_cell_rare(const CellArgs *ap, P *q, long long 
 {
     const CellArgs &a = *ap;
     const long long fs = a.L.fs;
-    const double dt = a.scal[0], T = a.T[c];
+    const double T = a.T[c];
     double cs[NV], CMS[NS], MD[NS];
     load_cs(a.cs, fs, c, cs);
     imex_source_t<false>(cs, T, a.quirks, CMS, MD, true);
-#pragma unroll
-    for (int v = 0; v < NV; v++) {
-        const double r = rhs_at<P>(a, v * fs + c);
-        cs[v] = v < NS ? cs[v] + (r + CMS[v] * dt) / (1.0 - dt * MD[v]) : cs[v] + r;
-    }
+    imex_update<P, false>(a, c, cs, CMS, MD);
     Decoded o;
     int capped = 0;
     decode(cs, T, (a.quirks & EU3D_Q_STALE_E) ? a.E[c] : 0.0, a.quirks, o, capped);
@@ -773,7 +810,7 @@ __device__ __forceinline__ void cell_body(const CellArgs &a, P *__restrict__ q, 
         }
         double CMS[NS], MD[NS];
         imex_source_t<SPEC>(cs, T, qk, CMS, MD, true);
-        imex_update<P>(a, c, cs, CMS, MD);
+        imex_update<P, SPEC>(a, c, cs, CMS, MD);
         decode(cs, T, Eold, qk, o, capped);
         capped_any |= capped;
         // a cell outside the specialised rates' range does it again, whole and
