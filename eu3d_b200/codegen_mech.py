@@ -176,10 +176,11 @@ def gen(mech) -> str:
 
     # IMEX: Diagonalized (R_TB defaults to 1)
     w("// Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s).  For T in")
-    w("// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in")
-    w("// the normal range (common.cuh's div_rn); the caller takes the table-driven")
-    w("// form elsewhere.")
-    w("constexpr double FAST_T_LO = 150.0, FAST_T_HI = 1e4;")
+    w("// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in the")
+    w("// range in which common.cuh's round as IEEE's (at 90 K equilibrium constants from")
+    w("// 1e-134 to 1e282 and backward rates above 1e-264); the caller takes the")
+    w("// table-driven form elsewhere.")
+    w("constexpr double FAST_T_LO = 90.0, FAST_T_HI = 1e4;")
     w("__device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[NS], const double Mc[NS],")
     w("                                                  const double Di[NS], const double PT[NS], double CMS[NS],")
     w("                                                  double MD[NS])")

@@ -323,8 +323,14 @@ __device__ __forceinline__ void warp_sum(unsigned long long *ctr, unsigned long 
 // scheduler from overlapping the 33 exponentials.  1.3 M cells: IMEX 0.85 ->
 // 0.40 ms (cold flow) and 0.69 -> 0.41 (hot), the adaptive chemistry on hot
 // gas 27.9 -> 16.5 ms.  Every other cell (and every other mechanism) takes the
-// table-driven form: below 150 K and above 1e4 K an equilibrium constant may
-// leave the range in which the quotients round as IEEE's.
+// table-driven form: colder and hotter an equilibrium constant may leave the range
+// in which the quotients round as IEEE's.  That form is slow, so the range reaches
+// down to 90 K, where the thermodynamic fits have long ended.  IMEX and adaptive
+// step of a gas between 108 and 208 K: 0.32 and 28 ms; with the range from 150 K
+// 4.7 and 483, with compiler divisions at every T 0.56 and 46.  Between 64 and 123
+// K: 5.0 and 1020 ms against 0.70 and 89.  (The specialised rates with IEEE quotients
+// out of line there take 1.2 and 272 ms but cost every cell 3 % of IMEX and 10 % of
+// the adaptive kernel.)
 template <bool FAST>
 __device__ __forceinline__ void imex_source_t(const double cs[NV], double T, unsigned qk, double CMS[NS], double MD[NS],
                                               bool tcouple)

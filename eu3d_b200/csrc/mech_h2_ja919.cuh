@@ -179,10 +179,11 @@ __device__ __forceinline__ void thermo_spec(const TPow &p, double h[NS], double 
 }
 
 // Reaction::Diagonalized per cell: CMS (kg/m^3/s) and MD(s, s).  For T in
-// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in
-// the normal range (common.cuh's div_rn); the caller takes the table-driven
-// form elsewhere.
-constexpr double FAST_T_LO = 150.0, FAST_T_HI = 1e4;
+// [FAST_T_LO, FAST_T_HI], where every rate constant and its quotients are in the
+// range in which common.cuh's round as IEEE's (at 90 K equilibrium constants from
+// 1e-134 to 1e282 and backward rates above 1e-264); the caller takes the
+// table-driven form elsewhere.
+constexpr double FAST_T_LO = 90.0, FAST_T_HI = 1e4;
 __device__ __forceinline__ void diagonalized_spec(const TPow &p, const double G[NS], const double Mc[NS],
                                                   const double Di[NS], const double PT[NS], double CMS[NS],
                                                   double MD[NS])

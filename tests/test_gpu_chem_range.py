@@ -1,15 +1,19 @@
 """Where the chemistry's straight-line quotients stop and IEEE division takes
-over: the adaptive integrator on both sides of 150 K and 1e4 K (a cell outside
+over: the adaptive integrator on both sides of 90 K and 1e4 K (a cell outside
 takes the table-driven rates and IEEE quotients, in one launch whose warps mix
-both), one-step IMEX at densities below 1e-30, and a mechanism other than the
+both), one-step IMEX on both sides of 90 K and at densities below 1e-30, the
+bits of cold cells within the range, and a mechanism other than the
 compiled-in one, whose rates are unbounded: its implicit update divides by
 denominators past the largest number and must give what the oracle gives, an
 update of zero, and not a NaN.
 
 Tolerances: one IMEX call 1e-12 of each variable's largest magnitude, the
 repository's bar; an adaptive step 1e-8, its bar against the oracle (the two
-sum in different orders, and a substep's length follows the state)."""
+sum in different orders, and a substep's length follows the state).  Cold
+cells: golden/cold_chem.npz holds what an implementation with the compiler's
+divisions recorded on a B200, whose bits the straight-line quotients give."""
 import copy
+import os
 
 import numpy as np
 import pytest
@@ -30,7 +34,9 @@ def _grid():
     return make_grid(33, 0.0, 0.01, 5, 0.0, 0.006, 3, 0.0, 0.004, 2, fixed_ghosts=True)
 
 
-WINDOWS = {"cold": (120.0, 190.0, 1e-12), "hot": (9700.0, 10300.0, 1e-13), "edge": (149.9, 150.1, 1e-12)}
+LOW, HIGH = 90.0, 1e4
+WINDOWS = {"cold": (80.0, 120.0, 1e-12), "hot": (9700.0, 10300.0, 1e-13), "edge": (89.9, 90.1, 1e-12)}
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "cold_chem.npz")
 
 
 @pytest.mark.parametrize("generic", [False, True], ids=["compiled-in", "table"])
@@ -45,7 +51,7 @@ def test_adaptive_outside_the_fast_range(mech, window, generic, monkeypatch):
     o.update_after_cs()
     d.update_after_cs()
     T = interior(o.view("T"))
-    assert (T < 150.0).any() or (T > 1e4).any()
+    assert ((T < LOW) | (T > HIGH)).any() and ((T > LOW) & (T < HIGH)).any()
     o.view("RHS")[...] = 0.0
     d.upload("RHS", np.zeros(d.shape("RHS")))
     d.set_elements(S.atoms_matrix(mech))
@@ -60,6 +66,52 @@ def test_adaptive_outside_the_fast_range(mech, window, generic, monkeypatch):
     # a rounding may move a substep boundary of a cell
     assert abs(st["substeps"] - int(n.sum())) <= 0.01 * n.sum()
     d.close()
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("window", ["cold", "edge"])
+def test_imex_around_the_lower_end(mech, window, bits):
+    lo, hi, dt = WINDOWS[window]
+    o, g = make_oracle(mech, seed=6, quirks=QUIRKS_FIXED, grid=_grid(), tlo=lo, thi=hi, radicals=1e-6)
+    d = gpu.DeviceFlowfield(mech, g, quirks=QUIRKS_FIXED, flux_bits=bits)
+    d.upload_state(o)
+    o.update_after_cs()
+    d.update_after_cs()
+    T = interior(o.view("T"))
+    assert (T < LOW).any() and (T > LOW).any()
+    o.partial_t()
+    o.dt = d.dt = dt
+    o.imex()
+    d.imex()
+    for f in ("CS", "T"):
+        e = rel_err(interior(d.download(f)), interior(o.view(f)))
+        assert e < TOL_FN, (f, e)
+    d.close()
+
+
+def cold_chemistry(mech):
+    """CS and T of cells between 92 and 170 K after one IMEX and one adaptive step."""
+    out = {}
+    for react in ("imex", "adaptive"):
+        g = make_grid(33, 0.0, 0.01, 3, 0.0, 0.006, 2, 0.0, 0.004, 2, fixed_ghosts=True)
+        o, g = make_oracle(mech, seed=8, quirks=QUIRKS_FIXED, grid=g, tlo=92.0, thi=170.0, radicals=1e-4)
+        d = gpu.DeviceFlowfield(mech, g, quirks=QUIRKS_FIXED, flux_bits=64)
+        d.upload_state(o)
+        d.update_after_cs()
+        d.upload("RHS", np.zeros(d.shape("RHS")))
+        d.set_elements(S.atoms_matrix(mech))
+        d.dt = 1e-8
+        d.imex() if react == "imex" else d.react_adaptive()
+        out[react] = np.concatenate([interior(d.download("CS")), interior(d.download("T"))[..., None]], axis=-1)
+        d.close()
+    return out
+
+
+def test_cold_cells_keep_the_bits_of_plain_divisions(mech):
+    got, want = cold_chemistry(mech), np.load(GOLDEN)
+    for react, v in got.items():
+        assert want[react][..., -1].min() > LOW and (want[react][..., -1] < 150.0).any()
+        assert np.array_equal(v, want[react]), react
 
 
 def test_imex_of_a_thin_gas(mech):
