@@ -1081,9 +1081,10 @@ struct SurSrcFieldApply : SurSrcField<P> {
 // Two resident blocks (255 registers): at three the substep loop spills 770
 // bytes a thread, and the cells' uneven substep counts leave little for the third
 // block to hide (272 against 226 us on 4.2 M cells of a developed oblique
-// detonation, 318 at four).
+// detonation, 318 at four).  The table-driven rates spill 32 bytes at three and
+// wait on their tables: three blocks (1.3 M hot cells 58 ms, 70 at two).
 template <class P, bool SPEC>
-__global__ void __launch_bounds__(128, 2) k_sur_fallback(CellArgs a, P *__restrict__ q, SurQueue qu)
+__global__ void __launch_bounds__(128, SPEC ? 2 : 3) k_sur_fallback(CellArgs a, P *__restrict__ q, SurQueue qu)
 {
     const int lane = threadIdx.x & 31;
     const int total = (int)min((long long)*qu.count, qu.cap);

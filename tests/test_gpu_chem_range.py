@@ -114,6 +114,27 @@ def test_cold_cells_keep_the_bits_of_plain_divisions(mech):
         assert np.array_equal(v, want[react]), react
 
 
+def test_queue_of_the_table_form_matches_thread_per_cell(mech, monkeypatch):
+    """The persistent queue, compiled for other resident blocks with the table-driven
+    rates, against one thread per cell: the same substeps, the state to rounding."""
+    monkeypatch.setenv("EU3D_GENERIC_CHEM", "1")
+    o, g = make_oracle(mech, seed=13, quirks=QUIRKS_FIXED, grid=_grid(), tlo=1100.0, thi=2600.0, radicals=1e-4)
+    out = []
+    for q in (0, 1):
+        d = gpu.DeviceFlowfield(mech, g, quirks=QUIRKS_FIXED, flux_bits=64)
+        d.upload_state(o)
+        d.upload("RHS", np.zeros(d.shape("RHS")))
+        d.set_elements(S.atoms_matrix(mech))
+        d.set_tuning(adapt_queue=q)
+        d.dt = 3e-8
+        d.react_adaptive()
+        out.append((d.status()["substeps"], {f: interior(d.download(f)) for f in ("CS", "T", "P")}))
+        d.close()
+    assert out[0][0] == out[1][0] > 33 * 5 * 3
+    for f, v in out[0][1].items():
+        assert rel_err(out[1][1][f], v) < TOL_FN, f
+
+
 def test_imex_of_a_thin_gas(mech):
     o = Oracle(mech, _grid(), QUIRKS_FIXED)
     fill_state(o, 6, 1100.0, 1500.0)
