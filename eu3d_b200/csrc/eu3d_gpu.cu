@@ -399,6 +399,25 @@ bool make_prim_map(eu3d_handle *h)
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// blocks of the FP64 flux with 32 x 7 tiles and walks of kz planes
+long long flux64_blocks(const Layout &L, int kz)
+{
+    return (long long)((L.ni + FT_X - 1) / FT_X) * ((L.nj + 6) / 7) * ((L.nk + kz - 1) / kz);
+}
+
+// z planes a block of the FP64 flux walks: the setting flux_kz, halved while the
+// tiles leave fewer than two waves of two blocks an SM, down to one plane.  A
+// walk of 16 already hides its extra z face (240 x 256 x 200: 2.32 ms, 2.43 with
+// 4 planes, 2.91 with 1); on smaller grids the blocks count for more (160^3: 0.75
+// ms with 4, 0.77 with 16; 121 x 81 x 61: 139 us with 2 or 4, 155 with 1; 241 x 81
+// x 2: 17.3 us with 1, 21.0 with 2).  Taken at the launch, so that no setting, the
+// autotuner's candidates among them, leaves a small grid to a few long walks.
+int flux64_walk(const Layout &L, int kz)
+{
+    while (kz > 1 && flux64_blocks(L, kz) < 2LL * 2 * 148) kz /= 2;
+    return kz;
+}
+
 // FP64 flux launch: tiles of 32 x 7 columns, two blocks of 8 warps per SM (128
 // registers a thread) where the grid fills the GPU; where it does not, 32 x 3
 // tiles, whose shorter blocks spread over more SMs (on a cheaper limiter, 7 -> 3
@@ -406,10 +425,9 @@ bool make_prim_map(eu3d_handle *h)
 // 160^3 0.56 -> 0.60 ms; with this one 17.3, 13.1 us and 0.75 ms, from 86.6, 78.4
 // us and 6.4 ms before the division-free faces).
 template <int DIFF, bool SQ, int TY, int NB>
-void launch_flux64(eu3d_handle *h, const FluxSolid &wedge)
+void launch_flux64(eu3d_handle *h, const FluxSolid &wedge, int kz)
 {
     const Layout &L = h->L;
-    const int kz = h->flux_kz;
     FieldBase qf;
     for (int f = 0; f < NPRIM; f++) qf.p[f] = (const char *)((const double *)h->prim + f * L.fs);
     const dim3 g((L.ni + FT_X - 1) / FT_X, (L.nj + TY - 1) / TY, (L.nk + kz - 1) / kz);
@@ -426,11 +444,11 @@ void launch_adv_t(eu3d_handle *h)
     const FluxSolid wedge{h->wedge[0], h->wedge[1], h->wedge[2], h->wedge_on};
     ProfScope ps(h, "advection");
     if constexpr (sizeof(P) == 8) {
-        const long long blocks = (long long)((L.ni + FT_X - 1) / FT_X) * ((L.nj + 6) / 7) * ((L.nk + kz - 1) / kz);
-        if (blocks < 2 * 148)
-            sq ? launch_flux64<DIFF, true, 3, 4>(h, wedge) : launch_flux64<DIFF, false, 3, 4>(h, wedge);
+        const int kw = flux64_walk(L, kz);
+        if (flux64_blocks(L, kw) < 2 * 148)
+            sq ? launch_flux64<DIFF, true, 3, 4>(h, wedge, kw) : launch_flux64<DIFF, false, 3, 4>(h, wedge, kw);
         else
-            sq ? launch_flux64<DIFF, true, 7, 2>(h, wedge) : launch_flux64<DIFF, false, 7, 2>(h, wedge);
+            sq ? launch_flux64<DIFF, true, 7, 2>(h, wedge, kw) : launch_flux64<DIFF, false, 7, 2>(h, wedge, kw);
     } else {
         const float *qf = (const float *)h->prim;
         if (h->flux_stage == 2 && h->tq_ok) {
@@ -1075,17 +1093,7 @@ int eu3d_create(const eu3d_desc *d, eu3d_handle **out)
         const long long cols = (long long)((L.ni + 31) / 32) * ((L.nj + 7) / 8);
         int kz = 64;
         while (kz > 4 && cols * ((L.nk + kz - 1) / kz) < 4LL * 2 * 148) kz /= 2;
-        if (d->flux_bits == 64) {
-            // FP64: a walk of 16 planes already hides its extra z face (240 x
-            // 256 x 200: 2.32 ms, 2.43 with 4 planes, 2.91 with 1); shorter
-            // ones while the 32 x 7 tiles leave fewer than two waves, down to
-            // one plane (160^3: 0.75 ms with 4, 0.77 with 16; 121 x 81 x 61:
-            // 139 us with 2 or 4, 155 with 1; 241 x 81 x 2: 17.3 us with 1,
-            // 21.0 with 2)
-            const long long c7 = (long long)((L.ni + 31) / 32) * ((L.nj + 6) / 7);
-            kz = 16;
-            while (kz > 1 && c7 * ((L.nk + kz - 1) / kz) < 2LL * 2 * 148) kz /= 2;
-        }
+        if (d->flux_bits == 64) kz = 16;  // at most (flux64_walk)
         h->flux_kz = kz;
     }
     if ((long long)NPRIM * L.fs >= (1LL << 31)) {
@@ -2212,7 +2220,8 @@ int eu3d_autotune(eu3d_handle *h, const eu3d_step_desc *s, int steps, eu3d_tunin
         }
     };
     copy(true);
-    std::vector<eu3d_tuning> cands;
+    // the setting the handle has comes first: the best is never a slower one
+    std::vector<eu3d_tuning> cands{start};
     const bool q = s->react == EU3D_REACT_TRAPEZOID && s->type == 1;
     const bool aq = s->react == EU3D_REACT_ADAPTIVE;
     for (int fst : {0, 1, 2})

@@ -301,7 +301,9 @@ int eu3d_sdlb_guest(eu3d_handle *h, int nseg, const long long *seg_cells, const 
 int eu3d_sdlb_unpack(eu3d_handle *h, const double *dev_back);
 
 /* Launch settings picked per handle (new): z planes walked by one flux block
-   (default: 64, halved while the flux grid has fewer than four waves),
+   (default: 64, halved while the flux grid has fewer than four waves; FP64
+   flux: 16, a limit that each launch halves while its tiles leave fewer than
+   two waves),
    adaptive trapezoid on the persistent work queue (1) or one thread per cell
    (0), resident queue blocks per SM, and how the FP32 flux kernel reads the
    primitives: 2 (default) tile planes brought into a shared-memory ring by
@@ -340,8 +342,8 @@ int eu3d_set_tuning(eu3d_handle *h, const eu3d_tuning *t);
    step graphs. */
 int eu3d_set_wait_limit(eu3d_handle *h, long long tries);
 int eu3d_get_tuning(eu3d_handle *h, eu3d_tuning *t);
-/* Autotuner: times `steps` steps of s for each candidate setting (flux_kz in
-   {4, 8, 16, 32, 64}, the three FP32 flux kernels; for the adaptive
+/* Autotuner: times `steps` steps of s for the present setting and each
+   candidate (flux_kz in {4, 8, 16, 32, 64}, the three FP32 flux kernels; for the adaptive
    trapezoid also the queue on/off and 2..4 blocks per SM; for the FP64
    adaptive chemistry adapt_queue on/off) on the handle's current state,
    restoring the state after each trial, and keeps the fastest.  best / best_ms may be NULL.  Needs
