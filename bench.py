@@ -70,7 +70,7 @@ def parse():
     ap.add_argument("--no-accuracy", action="store_true")
     ap.add_argument("--no-all-fp64", action="store_true", help="skip the all-FP64 IMEX arm of the headline")
     ap.add_argument("--tuning", default="",
-                    help="fixed launch settings instead of the autotuner, e.g. flux_kz=64,cell_blocks=4")
+                    help="fixed launch settings instead of the autotuner, e.g. flux_kz=64,flux_stage=2")
     ap.add_argument("--accuracy-steps", type=int, default=2000)
     ap.add_argument("--accuracy-full", action="store_true",
                     help="also compare on the benchmark's full grid (about 2.5 more minutes)")
