@@ -408,10 +408,11 @@ long long flux64_blocks(const Layout &L, int kz)
 // z planes a block of the FP64 flux walks: the setting flux_kz, halved while the
 // tiles leave fewer than two waves of two blocks an SM, down to one plane.  A
 // walk of 16 already hides its extra z face (240 x 256 x 200: 2.32 ms, 2.43 with
-// 4 planes, 2.91 with 1); on smaller grids the blocks count for more (160^3: 0.75
-// ms with 4, 0.77 with 16; 121 x 81 x 61: 139 us with 2 or 4, 155 with 1; 241 x 81
-// x 2: 17.3 us with 1, 21.0 with 2).  Taken at the launch, so that no setting, the
-// autotuner's candidates among them, leaves a small grid to a few long walks.
+// 4 planes, 2.90 with 1); on smaller grids the blocks count for more (160^3: 0.75
+// ms with 4, 0.77 with 16; 121 x 81 x 61: 137 us with 2 or 4, 154 with 1, 178 with
+// 16; 241 x 81 x 2: 15.4 us with 1, 19.7 with 2; 4000 x 2 x 2: 12.6, 16.7).  Taken
+// at the launch, so that no setting, the autotuner's candidates among them, leaves
+// a small grid to a few long walks.
 int flux64_walk(const Layout &L, int kz)
 {
     while (kz > 1 && flux64_blocks(L, kz) < 2LL * 2 * 148) kz /= 2;
@@ -419,11 +420,12 @@ int flux64_walk(const Layout &L, int kz)
 }
 
 // FP64 flux launch: tiles of 32 x 7 columns, two blocks of 8 warps per SM (128
-// registers a thread) where the grid fills the GPU; where it does not, 32 x 3
-// tiles, whose shorter blocks spread over more SMs (on a cheaper limiter, 7 -> 3
-// rows: 241 x 81 x 2 15.2 -> 13.1 us a launch, 4000 x 2 x 2 15.0 -> 11.2, but
-// 160^3 0.56 -> 0.60 ms; with this one 17.3, 13.1 us and 0.75 ms, from 86.6, 78.4
-// us and 6.4 ms before the division-free faces).
+// registers a thread) where the grid fills the GPU; where it leaves less than a
+// wave of them, 32 x 3 tiles, whose shorter blocks spread over more SMs.  7 and 3
+// rows, us a launch: 4000 x 2 x 2 16.7, 12.6; 241 x 81 x 2 18.6, 15.7; 64 x 64 x 40
+// 44.4, 43.2 (above the line); 121 x 81 x 61 138, 141; 512 x 256 x 2 64.5, 80.2;
+// 160^3 777, 860.  (78, 87 us and 5.0 to 6.4 ms before the division-free faces, first
+// two and last.)
 template <int DIFF, bool SQ, int TY, int NB>
 void launch_flux64(eu3d_handle *h, const FluxSolid &wedge, int kz)
 {

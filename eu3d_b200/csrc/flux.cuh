@@ -398,15 +398,15 @@ constexpr int FT_X = 32;
 // order ((-dt/dx dF - dt/dy dG) - dt/dz dQ).
 // Cells are read through L1: the four planes a z face spans and the tile's
 // halo are re-read from L1 and L2, whose bandwidth is not the bound (232 B a
-// cell of HBM traffic).  What bounds it is the FP64 pipe together with issue
-// and latency: 3780 warp instructions a cell, 1710 of them FP64 (two cycles
-// each), at 16 warps an SM (128 registers).  160^3: 0.75 ms a launch; 6.4 ms
-// with the compiler's quotients (16 000 instructions a cell, an FP64 pipe 12 %
-// busy behind branches, barriers and instruction fetches).  Left out, measured
-// on a cheaper form of the limiter: three inlined copies of the face (0.77 ms
-// against 0.62: instruction cache), 96 registers and 20 warps (0.77), an L2
-// prefetch of plane k + 3 (0.58 against 0.56), per-load address products
-// instead of field bases in the constant bank (0.62 against 0.56).
+// cell of HBM traffic).  What bounds it is latency with too few warps to hide it:
+// 3780 warp instructions a cell, 1710 of them FP64 (two cycles each), at 16 warps
+// an SM (128 registers) keep the FP64 pipe 45 % and the issue slots 53 % busy; of
+// a warp's 7.2 cycles an instruction 1.9 wait for loads, 1.6 are fixed latencies,
+// 0.8 barriers, 0.5 the FP64 pipe (160 x 128 x 96, 0.41 ms).  160^3: 0.78 ms a
+// launch; 5.0 to 6.4 ms with the compiler's quotients (16 000 instructions a cell,
+// an FP64 pipe 12 % busy behind branches, barriers and instruction fetches).  Left
+// out, 160^3 in ms: three inlined copies of the face 0.84 (instruction cache); 20
+// warps at 96 registers 1.26 (spills); an L2 prefetch four planes ahead 0.80.
 template <int TY>
 struct Flux64 {
     static constexpr int THREADS = FT_X * (TY + 1);

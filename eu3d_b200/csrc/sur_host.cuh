@@ -123,8 +123,9 @@ SurBf16 sur_bf16(const eu3d_surrogate *s)
 void sur_train_step(eu3d_surrogate *s, float *out4, float *loss, const AdamCfg &adam, const BatchSrc &next, const SurNorm &nrm)
 {
     const int grid = sur_train_grid(s, s->B);
-    k_sur_train<<<grid, TRN_THREADS, TrainSmem::BYTES + 128, s->st>>>(s->Xb, s->Yb, sur_bf16(s), s->p, s->zbuf, s->part,
-                                                                     out4, s->B, s->dzt, s->err);
+    auto train = s->dzt ? k_sur_train<true> : k_sur_train<false>;
+    train<<<grid, TRN_THREADS, TrainSmem::BYTES + 128, s->st>>>(s->Xb, s->Yb, sur_bf16(s), s->p, s->zbuf, s->part, out4,
+                                                               s->B, s->dzt, s->err);
     if (s->dzt) k_sur_bias<<<3 * SUR_H + SUR_OUT, TRN_CHUNK, 0, s->st>>>(s->dzt, s->B, s->part);
     const int blocks = STEP_BLOCKS + (int)(((long long)next.B * BATCH_TASKS + 255) / 256);
     k_sur_step<<<blocks, 4 * STEP_PARAMS, 0, s->st>>>(s->part, grid, s->p, s->m, s->v, adam.update ? nullptr : s->g, loss,
@@ -180,7 +181,8 @@ int sur_set_attrs()
 {
     static bool done = false;
     if (done) return EU3D_OK;
-    CK(cudaFuncSetAttribute(k_sur_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TrainSmem::BYTES + 128));
+    for (auto k : {k_sur_train<false>, k_sur_train<true>})
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TrainSmem::BYTES + 128));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcArray>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcField<float>>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));
     CK(cudaFuncSetAttribute(k_sur_mlp<SurSrcField<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, SURK_SMEM));

@@ -128,9 +128,11 @@ __device__ __forceinline__ float trn_colsum(const unsigned char *tr, int c, int 
 }
 
 // Xb, Yb: features and targets of the batch, B x 16 each (column 15 of Yb the
-// sample's weight).  dzt: null, and block b takes the tiles b, b + gridDim.x,
-// ...; or (trn_paired) the place of dZ_l^T, [4][128][B], and block b takes the
-// tiles 2 b and 2 b + 1 and leaves the bias gradients to k_sur_bias.
+// sample's weight).  Block b takes the tiles b, b + gridDim.x, ...; PAIRED
+// (trn_paired): the tiles 2 b and 2 b + 1, and it leaves dZ_l^T in dzt ([4][128][B])
+// for k_sur_bias instead of summing the bias gradients.  A template, since the
+// choice at run time costs the large batches 3 % (44 against 45.5 us a step).
+template <bool PAIRED>
 __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__restrict__ Xb, const float *__restrict__ Yb,
                                                              SurBf16 w, const float *__restrict__ p,
                                                              float *__restrict__ zbuf,
@@ -227,14 +229,14 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
         trn_store_tile(sm + S::ACT, sm + tr, row, c0, h);
     };
     float *ys = reinterpret_cast<float *>(sm + S::YS);
-    const int tile_step = dzt ? 1 : gridDim.x, tile_end = dzt ? 2 * blockIdx.x + 2 : B / 128;
+    const int tile_step = PAIRED ? 1 : gridDim.x, tile_end = PAIRED ? 2 * blockIdx.x + 2 : B / 128;
     // bias gradient of layer l (0-based) from the tile of dZ^T in T3
     auto bias_grad = [&](int l, int tile) -> float {
-        if (!dzt) return trn_colsum(sm + S::T3, tid & 127, quarter);
+        if (!PAIRED) return trn_colsum(sm + S::T3, tid & 127, quarter);
         trn_copy_col(dzt + (size_t)(l * SUR_H + (tid & 127)) * B + tile * 128 + 32 * quarter, sm + S::T3, tid & 127, quarter);
         return 0.f;
     };
-    for (int tile = dzt ? 2 * blockIdx.x : blockIdx.x; tile < tile_end; tile += tile_step) {
+    for (int tile = PAIRED ? 2 * blockIdx.x : blockIdx.x; tile < tile_end; tile += tile_step) {
         const long long r = (long long)tile * 128 + row;
         float wt = 0.f;
         if (quarter == 0) {
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
             if (l == 2) {
                 // column tid & 15, rows 4 (tid >> 4) .. + 3
                 const uint2 x = *reinterpret_cast<const uint2 *>(sm + S::DZ4T + tc::op_off(16, tid & 15, 4 * (tid >> 4)));
-                if (dzt)
+                if (PAIRED)
                     *reinterpret_cast<uint2 *>(dzt + (size_t)(3 * SUR_H + (tid & 15)) * B + tile * 128 + 4 * (tid >> 4)) = x;
                 else
                     db4 += (__uint_as_float(x.x << 16) + __uint_as_float(x.x & 0xffff0000u)) +
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(TRN_THREADS, 1) k_sur_train(const float *__res
 // 4e-8 to 6e-6 at 1024 to 3072 rows where 128-row partials differ by 5e-6 to
 // 2e-5, and at 4096 rows both differ by 4e-6.  From there on a block takes 128
 // rows, which keeps twice the SMs busy: 43 us a step against 82 at 4096 and 8192
-// rows (below 4096 rows 39 to 41 against the 78 to 81 us of this order).
+// rows (below 4096 rows 39 to 43 against the 76 to 84 us of this order).
 constexpr int TRN_CHUNK = 256, TRN_CHUNKS = 16;
 __host__ __device__ constexpr bool trn_paired(int B) { return B < TRN_CHUNKS * TRN_CHUNK; }
 
