@@ -16,7 +16,7 @@
 // time; as some 30 kernels (a GEMM, an activation, a column sum, ... per
 // layer) it took 480 us, each kernel a chain of global round trips: transposed
 // activations in 2-byte scattered stores, uncoalesced GEMM epilogues and 32
-// blocks of atomics per weight gradient.  Now 45 us: 33 for this kernel, 10 for
+// blocks of atomics per weight gradient.  Now 43 us: 33 for this kernel, 10 for
 // the second, which also makes the next batch (FP64 targets; inside this
 // kernel they took 5 us of its chain).  What bounds it is a tile's chain of
 // eight tensor-core waits (1100 to 2000 cycles each) with an epilogue between
